@@ -8,7 +8,7 @@ tests and benchmark (32 query heads over 8 KV heads, their eighth for one rank o
 over 32; groups of 2, 3 and 8; windows of 576 and 1000; 64 x 64 and 128 x 128 latents with 24 heads).
 
 `listed()` names the cases, `draw()` gives more of the same ranges, `prepare()` makes the tensors a
-program holds before the call, `run()` is one pass.
+program holds before the call, `run()` is one pass, `exact()` the same attention in 64 bits.
 """
 import math
 
@@ -201,3 +201,77 @@ def tolerance(case):
     # same inputs, over decode, every causal and image pattern: rel 1.9e-3 .. 2.4e-3, max 6e-3 .. 3.3e-2
     # (log-sum-exp: 4e-7); about four times that.
     return {"rel": 1e-2, "max": 0.12}
+
+
+def _attend(q, k, v, rows, keys, visible=None, lse=None):
+    """64-bit attention of the query tokens `rows` over the key tokens `keys`; tensors are (B, H, S, D)."""
+    rep = q.shape[1] // k.shape[1]
+    out = torch.empty(q.shape[0], q.shape[1], len(rows), HEAD_DIM, dtype=torch.float64, device=q.device)
+    for b in range(q.shape[0]):
+        for hk in range(k.shape[1]):
+            kk, vv = k[b, hk, keys].double(), v[b, hk, keys].double()
+            heads = slice(hk * rep, (hk + 1) * rep)
+            s = q[b, heads][:, rows].double() @ kk.T * HEAD_DIM ** -0.5
+            if visible is not None:
+                s.masked_fill_(~visible, float("-inf"))
+            if lse is not None:
+                lse[b, heads, rows] = s.logsumexp(-1)
+            out[b, heads] = s.softmax(-1) @ vv
+    return out
+
+
+def exact(case, seed):
+    state = prepare(case, seed)
+    q, k, v = state["qkv"]
+    call = case["call"]
+    if call == "decode":
+        out = torch.empty(q.shape, dtype=torch.float64, device="cuda")
+        for b in range(case["B"]):
+            keys = torch.arange(case["S"], device="cuda")
+            keys = keys if state["mask"] is None else keys[state["mask"][b, 0, 0]]
+            one = slice(b, b + 1)
+            out[one] = _attend(q[one], k[one], v[one], torch.zeros(1, dtype=torch.long, device="cuda"), keys)
+        return out.transpose(1, 2)
+    if call == "llm":
+        q, k, v = (x.transpose(1, 2) for x in (q, k, v))
+    S = q.shape[2]
+    pattern = case["pattern"]
+    token = torch.arange(S, device="cuda")
+    out = torch.empty(q.shape, dtype=torch.float64, device="cuda")
+    lse = torch.empty(q.shape[:3], dtype=torch.float64, device="cuda") if case.get("lse") else None
+
+    def attend(rows, keys, visible=None):
+        for part in rows.split(2048):                     # bounds the score matrix
+            seen = None if visible is None else visible(part[:, None], keys[None, :])
+            out[:, :, part] = _attend(q, k, v, part, keys, seen, lse)
+
+    if call == "image":
+        W = case["width"]
+        text, row, col = token[:TEXT_LEN], (token - TEXT_LEN) // W, (token - TEXT_LEN) % W
+        group = torch.where(token < TEXT_LEN, token // 64, row % 2 * 4 + col % 4)
+        for g in range(8):
+            members = (token >= TEXT_LEN) & (row % 2 * 4 + col % 4 == g)
+            rows = group == g if pattern == "scatter" else (token < TEXT_LEN) & (group == g)
+            attend(token[rows], torch.cat([text, token[members]]))
+        if pattern == "gather0":
+            def start(patch):                             # of the 16-wide window around an 8-wide patch
+                return min(max(patch * 8 - 4, 0), W - 16)
+            for r in range(W // 8):
+                for c in range(W // 8):
+                    near = (token >= TEXT_LEN) & (row >= start(r)) & (row < start(r) + 16) \
+                        & (col >= start(c)) & (col < start(c) + 16)
+                    patch = (token >= TEXT_LEN) & (row // 8 == r) & (col // 8 == c)
+                    attend(token[patch], torch.cat([text, token[near]]))
+        return out
+    param = case.get("param", 576 if pattern == "window" else 8)
+    if pattern == "window":
+        for first in range(0, S, 1024):
+            attend(token[first:first + 1024], token[max(0, first - param):first + 1024],
+                   lambda i, j: (j <= i) & (j >= i // 64 * 64 - (param - 64)))
+    else:
+        group = token % param if pattern == "scatter" else token // param % param
+        for g in range(param):
+            members = token[group == g]
+            attend(members, members, lambda i, j: j <= i)
+    out = out.transpose(1, 2)
+    return out if lse is None else (out, lse)
