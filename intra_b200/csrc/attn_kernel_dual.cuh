@@ -91,7 +91,7 @@ __device__ __forceinline__ void tma_fetch_tile(const Problem& prob, const Tile& 
                                                int batch, const TmaOperand& op, uint32_t dst, uint64_t* bar) {
   int c[5];
   const int is_text = tma_box_coords(prob, t, start, text, head, batch, c);
-  const bool rank4 = is_text || t.kind == KIND_LLM_WINDOW;
+  const bool rank4 = tma_rank4(t, is_text);
   // a Gather-0 problem's text tiles are image-Scatter tiles whose image keys come through the aux view
   const CUtensorMap* m = is_text ? op.text_map : (prob.kind == KIND_IMG_GATHER0 ? op.aux_map : op.main_map);
 #pragma unroll
@@ -200,7 +200,7 @@ struct KvSegment {
   int c[5];          // coordinates of the segment's first tile (c[0] unused)
   int d[5];          // increment per tile
   int first;         // first tile of the segment
-  int text;          // 1: text map (rank 4), 0: main / aux map
+  int text;          // 1: text map, 0: main / aux map
   int rank4;
 };
 __device__ __forceinline__ void kv_segment(const Problem& prob, const Tile& kv, int first, int n_kv, int head, int batch,
@@ -209,7 +209,7 @@ __device__ __forceinline__ void kv_segment(const Problem& prob, const Tile& kv, 
   tma_kv_start(kv, first, &start, &text);
   sg->first = first;
   sg->text = tma_box_coords(prob, kv, start, text, head, batch, sg->c);
-  sg->rank4 = sg->text || kv.kind == KIND_LLM_WINDOW;
+  sg->rank4 = tma_rank4(kv, sg->text);
   int c1[5];
   if (first + 1 < n_kv) {
     tma_kv_start(kv, first + 1, &start, &text);
@@ -258,7 +258,7 @@ __device__ __forceinline__ void plan_query(const Problem& prob, const Tile& t, i
   int start; bool text;
   tma_q_start(t, &start, &text);
   *is_text = tma_box_coords(prob, t, start, text, head, batch, c);
-  *rank4 = *is_text || t.kind == KIND_LLM_WINDOW;
+  *rank4 = tma_rank4(t, *is_text);
 }
 // TMA box coordinates of an item's two query tiles and of its key tiles (shared-key modes), for the
 // thread that issues the loads.

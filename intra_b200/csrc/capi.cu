@@ -167,10 +167,15 @@ bool build_maps(const Problem& p, const __nv_bfloat16* ptr, const TensorView& tv
   const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
   switch (p.kind) {
     case KIND_LLM_SCATTER: {
-      const cuuint64_t dims[5] = {128, cuuint64_t(p.G), cuuint64_t(p.S / p.G), cuuint64_t(heads), cuuint64_t(B)};
+      const int longer = p.n_longer;      // groups 0..longer-1 have one token more: a view of their own
+      cuuint64_t dims[5] = {128, cuuint64_t(p.G - longer), cuuint64_t(p.S / p.G), cuuint64_t(heads), cuuint64_t(B)};
       const cuuint64_t str[4] = {ss, ss * p.G, sh, sb};
       const cuuint32_t box[5] = {64, 1, 128, 1, 1};
-      return encode_map(main_map, ptr, 5, dims, str, box, ones);
+      if (!encode_map(main_map, ptr + int64_t(longer) * tv.ss, 5, dims, str, box, ones)) return false;
+      if (longer == 0) return true;
+      dims[1] = longer;
+      dims[2] += 1;
+      return encode_map(text_map, ptr, 5, dims, str, box, ones);
     }
     case KIND_LLM_GATHER1: {
       const cuuint64_t span = cuuint64_t(p.G) * p.G;

@@ -55,6 +55,7 @@ struct Problem {
   int tiles_m;  // scatter / gather1: tiles per group;  image scatter: tiles per group
   int n_img;    // image kinds: image tokens per group = W*W/8
   int pairs_per_row;  // gather0: patch pairs per patch row
+  int n_longer;       // scatter: the first S % G groups have one token more than the others
 };
 
 // Length of group g's packed token list for the two grouped LLM patterns.
@@ -83,7 +84,7 @@ INTRA_HD int gather0_start(int x, int np) {
 INTRA_HD int make_problem(int kind, int S, int G, int W, Problem* out) {
   Problem p;
   p.kind = kind; p.S = S; p.G = G; p.W = W;
-  p.n_tiles = 0; p.tiles_m = 0; p.n_img = 0; p.pairs_per_row = 0;
+  p.n_tiles = 0; p.tiles_m = 0; p.n_img = 0; p.pairs_per_row = 0; p.n_longer = 0;
   if (S <= 0) return -1;
   switch (kind) {
     case KIND_LLM_SCATTER:
@@ -91,6 +92,7 @@ INTRA_HD int make_problem(int kind, int S, int G, int W, Problem* out) {
       if (G <= 0 || G > S) return -1;
       int nmax = 0;
       for (int g = 0; g < G; ++g) nmax = imax(nmax, llm_group_len(kind, S, G, g));
+      if (kind == KIND_LLM_SCATTER) p.n_longer = S % G;
       p.tiles_m = ceil_div(nmax, TILE_M);
       p.n_tiles = p.tiles_m * G;
       break;
