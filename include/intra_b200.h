@@ -74,6 +74,24 @@ int intra_b200_fwd_image_lse(const void* q, const void* k, const void* v, void* 
                              int pattern, int width, float softmax_scale,
                              int device, void* cuda_stream);
 
+/* Dense attention of one new token per sequence over its KV cache, the decode step of the reference's
+ * attention backend (experiments/llm/intra_token_attn.py:112-134). Row (b, h) of q and out is 128 bf16
+ * values, out being contiguous (B, H, 128); k and v are B x S x Hkv rows of 128 by strides (in elements,
+ * multiples of 8; 0 repeats). `mask` is NULL or B x S bytes by strides (in bytes), nonzero = the key is
+ * visible; masked keys are not read, a sequence without a visible key gets zeros.
+ * Caches that are split over more CTAs than one thread-block cluster holds need scratch: when
+ * `scratch` is too small the call launches nothing, stores the bytes wanted in *scratch_needed and
+ * returns INTRA_NEED_SCRATCH; the buffer (device memory, 16-byte aligned) must stay untouched until the
+ * call's work on `cuda_stream` is done. Allocates nothing. */
+#define INTRA_NEED_SCRATCH 1
+int intra_b200_decode(const void* q, const void* k, const void* v, const void* mask, void* out, void* scratch,
+                      int64_t scratch_bytes, int64_t* scratch_needed, int B, int S, int H, int Hkv,
+                      int64_t q_batch_stride, int64_t q_head_stride,
+                      int64_t k_batch_stride, int64_t k_token_stride, int64_t k_head_stride,
+                      int64_t v_batch_stride, int64_t v_token_stride, int64_t v_head_stride,
+                      int64_t mask_batch_stride, int64_t mask_token_stride,
+                      float softmax_scale, int device, void* cuda_stream);
+
 /* Text for a status code; replaces the reference's TORCH_CHECK messages
  * (csrc/flash_attn/flash_api.cpp:377-394, 576-597). */
 const char* intra_b200_strerror(int status);

@@ -12,10 +12,11 @@ import os
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG_DIR, "_lib", "libintra_b200.so")
 
+NEED_SCRATCH = 1
 OK, ERR_BAD_ARG, ERR_UNSUPPORTED, ERR_ALIGNMENT, ERR_CUDA, ERR_DEVICE, ERR_KERNEL = 0, -1, -2, -3, -4, -5, -6
 
 _I64x3 = ctypes.POINTER(ctypes.c_int64)
-_vp, _i, _f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+_vp, _i, _f, _i64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_int64
 
 # name -> (restype, argtypes); every symbol include/intra_b200.h declares.
 SIGNATURES = {
@@ -29,6 +30,8 @@ SIGNATURES = {
                                       _i, _i, _f, _i, _vp]),
     "intra_b200_fwd_llm_noalloc": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _I64x3, _I64x3, _I64x3, _I64x3,
                                         _i, _i, _i, _f, _i, _vp, ctypes.POINTER(_i)]),
+    "intra_b200_decode": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, ctypes.POINTER(_i64), _i, _i, _i, _i,
+                               _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _f, _i, _vp]),
     "intra_b200_strerror": (ctypes.c_char_p, [_i]),
     "intra_b200_last_cuda_error": (_i, []),
     "intra_b200_device_status": (_i, [_i, ctypes.POINTER(_i), _i]),

@@ -15,6 +15,7 @@
 
 #include "attn_kernel.cuh"
 #include "attn_kernel_dual.cuh"
+#include "decode_kernel.cuh"
 #include "gather_kernel.cuh"
 #include "selftest.cuh"
 
@@ -375,9 +376,126 @@ int run_fwd(const void* q, const void* k, const void* v, void* out, int B, int S
                     g_dev[device].sm_count, static_cast<cudaStream_t>(stream), lse);
 }
 
+// ---- one-token decode --------------------------------------------------------------------------------
+struct DecodeState {
+  std::once_flag once;
+  int init_status = INTRA_OK;
+  int sm_count = 0;
+  int max_cluster = 8;            // 16 where the device can place such a cluster, else the portable 8
+};
+DecodeState g_decode[MAX_DEVICES];
+
+// Runs once per device with that device current. Allocates nothing, so a first call may be captured.
+void init_decode(int device) {
+  DecodeState& st = g_decode[device];
+  int major = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device);
+  if (e != cudaSuccess) { st.init_status = cuda_fail(e); return; }
+  if (major != 10) { st.init_status = INTRA_ERR_DEVICE; return; }
+  e = cudaDeviceGetAttribute(&st.sm_count, cudaDevAttrMultiProcessorCount, device);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = opt_in_smem(decode_kernel, DEC_SMEM_BYTES);
+  if (e != cudaSuccess) { st.init_status = cuda_fail(e); return; }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim = {16, 1, 1};
+  cfg.gridDim = dim3(16);
+  cfg.blockDim = dim3(DEC_THREADS);
+  cfg.dynamicSmemBytes = DEC_SMEM_BYTES;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int placed = 0;
+  if (cudaOccupancyMaxActiveClusters(&placed, decode_kernel, &cfg) == cudaSuccess && placed >= 8) st.max_cluster = 16;
+  else cudaGetLastError();        // not an error of the call: the portable size will do
+}
+
+// How a cache of S keys is dealt out: CTAs per cluster and clusters per unit (a batch entry's KV head with
+// up to 8 query heads). Measured over 1..256 units of 128..65536 keys (us, one launch in a CUDA graph):
+//   * as many CTAs as are resident at once (two per SM), with two key blocks each at least: 32 units of 4096
+//     keys 33 / 17.1 / 13.3 with 1 / 4 / 8 CTAs per unit; 256 units of 1024 keys 26.1 / 29.7 with 1 / 2;
+//   * more where a CTA would get more than DEC_MAX_BLOCKS blocks: 128 units of 8192 keys 83.8 with 4;
+//   * 16 CTAs per cluster only for few units (such a cluster needs 16 free places at once in a part of the
+//     chip) and where 8 leave too little in flight: 8 units of 4096 keys 9.6 against 10.9 with 8 and 10.1 with 4
+//     clusters of 8 and the merging launch, which costs 2 us. At 8192 keys it is 13.3 against 11.5: several clusters;
+//   * several clusters: up to the resident CTAs, 16 blocks per CTA at least: 1 unit of 16384 keys 10.0.
+void plan_decode(int64_t units, int S, int sm_count, int max_cluster, int* cluster, int* n_clusters) {
+  const int n_blk = ceil_div(S, DEC_BLOCK);
+  const int64_t slots = int64_t(sm_count) * DEC_CTAS_PER_SM;
+  int c = 1;
+  while (c < 8 && units * 2 * c <= slots && n_blk >= 4 * c) c *= 2;
+  while (c < 8 && n_blk > c * DEC_MAX_BLOCKS) c *= 2;
+  if (max_cluster >= 16 && units * 16 <= sm_count && n_blk >= 64 && n_blk < 512) c = 16;
+  int n = ceil_div(n_blk, c * DEC_MAX_BLOCKS);
+  if (c <= 8) {
+    const int64_t fits = slots / (units * c);
+    n = imax(n, imin(n_blk / (16 * c), fits < 4096 ? int(fits) : 4096));
+  }
+  *cluster = c;
+  *n_clusters = n;
+}
+
 }  // namespace
 
 extern "C" {
+
+int intra_b200_decode(const void* q, const void* k, const void* v, const void* mask, void* out, void* scratch,
+                      int64_t scratch_bytes, int64_t* scratch_needed, int B, int S, int H, int Hkv, int64_t q_batch_stride,
+                      int64_t q_head_stride, int64_t k_batch_stride, int64_t k_token_stride, int64_t k_head_stride,
+                      int64_t v_batch_stride, int64_t v_token_stride, int64_t v_head_stride, int64_t mask_batch_stride,
+                      int64_t mask_token_stride, float softmax_scale, int device, void* cuda_stream) {
+  if (!q || !k || !v || !out || !scratch_needed || B <= 0 || S <= 0 || H <= 0 || Hkv <= 0 || H % Hkv != 0)
+    return INTRA_ERR_BAD_ARG;
+  const int64_t strides = q_batch_stride | q_head_stride | k_batch_stride | k_token_stride | k_head_stride |
+                          v_batch_stride | v_token_stride | v_head_stride;
+  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out) || (strides & 7) != 0 || !aligned16(scratch))
+    return INTRA_ERR_ALIGNMENT;
+  if (device < 0 || device >= MAX_DEVICES) return INTRA_ERR_BAD_ARG;
+  DeviceGuard guard(device);
+  if (!guard.ok) return cuda_fail(cudaGetLastError());
+  DecodeState& st = g_decode[device];
+  std::call_once(st.once, init_decode, device);
+  if (st.init_status != INTRA_OK) return st.init_status;
+
+  DecodeParams p;
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.k = static_cast<const __nv_bfloat16*>(k);
+  p.v = static_cast<const __nv_bfloat16*>(v);
+  p.mask = static_cast<const uint8_t*>(mask);
+  p.o = static_cast<__nv_bfloat16*>(out);
+  p.scratch = static_cast<float*>(scratch);
+  p.q_sb = q_batch_stride; p.q_sh = q_head_stride;
+  p.ks = {k_batch_stride, k_token_stride, k_head_stride};
+  p.vs = {v_batch_stride, v_token_stride, v_head_stride};
+  p.mask_sb = mask_batch_stride; p.mask_ss = mask_token_stride;
+  p.mask_vec = mask && mask_token_stride == 1 && aligned16(mask) && mask_batch_stride % 16 == 0;
+  p.S = S; p.H = H; p.Hkv = Hkv;
+  p.head_groups = ceil_div(H / Hkv, DEC_HEADS);
+  p.scale_log2 = softmax_scale * 1.4426950408889634f;
+  const int64_t units = int64_t(B) * Hkv * p.head_groups;
+  plan_decode(units, S, st.sm_count, st.max_cluster, &p.cluster, &p.n_clusters);
+  const int64_t clusters = units * p.n_clusters;
+  if (clusters * p.cluster > 0x7fffffffLL || int64_t(B) * H > 0x7fffffffLL) return INTRA_ERR_UNSUPPORTED;
+  *scratch_needed = p.n_clusters > 1 ? clusters * DEC_PARTIAL * int64_t(sizeof(float)) : 0;
+  if (*scratch_needed > 0 && (!scratch || scratch_bytes < *scratch_needed)) return INTRA_NEED_SCRATCH;
+
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim = {unsigned(p.cluster), 1, 1};
+  cfg.gridDim = dim3(unsigned(clusters * p.cluster));
+  cfg.blockDim = dim3(DEC_THREADS);
+  cfg.dynamicSmemBytes = DEC_SMEM_BYTES;
+  cfg.stream = static_cast<cudaStream_t>(cuda_stream);
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, decode_kernel, p);
+  if (e == cudaSuccess && p.n_clusters > 1) {
+    decode_merge_kernel<<<unsigned(B) * unsigned(H), HEAD_DIM, 0, cfg.stream>>>(p);
+    e = cudaGetLastError();
+  }
+  return e == cudaSuccess ? INTRA_OK : cuda_fail(e);
+}
 
 int intra_b200_fwd_llm(const void* q, const void* k, const void* v, void* out, int B, int S, int H, int Hkv,
                        const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],

@@ -8,6 +8,8 @@ they divide the query heads. Forward only.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _loader
@@ -187,12 +189,63 @@ def intra_image_attn(q, k, v, pattern="scatter", width=64, softmax_scale=None, *
     return (out, lse) if return_lse else out
 
 
+def decode_attn(q, k, v, mask=None, softmax_scale=None):
+    """Dense attention of one token per sequence over its cache: q (B, H, 1, 128), k and v
+    (B, Hkv, S, 128), `mask` None or bool (B or 1, 1, 1, >= S), nonzero = visible. Returns (B, 1, H, 128), or None
+    for calls the decode kernel does not take - other types, devices, layouts or broadcasts, masks per
+    head or additive, and everything that looks inside an operator (autograd, forward-mode, vmap, tracing,
+    dispatch modes, autocast to another type) - which are the caller's to run as torch operators."""
+    if type(q) is not torch.Tensor or type(k) is not torch.Tensor or type(v) is not torch.Tensor:
+        return None
+    if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16 or not q.is_cuda:
+        return None
+    if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
+        return None
+    if (torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None
+            or torch._C._len_torch_dispatch_stack() or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch.autograd.forward_ad._current_level >= 0 or q.is_neg() or k.is_neg() or v.is_neg()
+            or (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.bfloat16)):
+        return None
+    dev = q.device
+    if q.dim() != 4 or k.dim() != 4 or k.shape != v.shape or k.device != dev or v.device != dev:
+        return None
+    B, H, n, D = q.shape
+    Bk, Hkv, S, Dk = k.shape
+    if n != 1 or D != 128 or Dk != 128 or Bk != B or B == 0 or S == 0 or Hkv == 0 or H < Hkv or H % Hkv:
+        return None
+    qs, ks, vs = q.stride(), k.stride(), v.stride()
+    qp, kp, vp = q.data_ptr(), k.data_ptr(), v.data_ptr()
+    if (qs[3] != 1 or ks[3] != 1 or vs[3] != 1 or (qp | kp | vp) & 15
+            or (qs[0] | qs[1] | ks[0] | ks[1] | ks[2] | vs[0] | vs[1] | vs[2]) & 7):
+        return None
+    mp, ms0, ms1 = None, 0, 0
+    if mask is not None:
+        if (type(mask) is not torch.Tensor or mask.dtype != torch.bool or mask.dim() != 4 or mask.device != dev
+                or mask.shape[0] not in (1, B) or mask.shape[1] != 1 or mask.shape[2] != 1 or mask.shape[3] < S):
+            return None
+        mp, ms0, ms1 = mask.data_ptr(), mask.stride(0) if mask.shape[0] == B else 0, mask.stride(3)
+    out = q.new_empty((B, 1, H, D))
+    need = ctypes.c_int64(0)
+    scratch, nbytes = None, 0
+    while True:
+        rc = lib.intra_b200_decode(qp, kp, vp, mp, out.data_ptr(), None if scratch is None else scratch.data_ptr(), nbytes,
+                                   need, B, S, H, Hkv, qs[0], qs[1], ks[0], ks[2], ks[1], vs[0], vs[2], vs[1], ms0, ms1,
+                                   0.08838834764831845 if softmax_scale is None else softmax_scale, dev.index,
+                                   torch._C._cuda_getCurrentRawStream(dev.index))
+        if rc != _loader.NEED_SCRATCH:
+            break
+        nbytes = need.value
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    if rc != 0:
+        _raise(rc)
+    return out
+
+
 def device_status(device=None, reset=False):
     """Synchronise `device` and return the status word its kernels write when a bounded wait gives
     up (0 = healthy; otherwise 100 + the id of the first wait that ran out since the last reset). The
     attention calls never poll it, and a recorded failure does not change later launches: a caller that
     wants to know checks here, e.g. once per step. Raises nothing; callers decide."""
-    import ctypes
     dev = torch.cuda.current_device() if device is None else torch.device(device).index
     word = ctypes.c_int(0)
     lib.intra_b200_device_status(dev, ctypes.byref(word), 1 if reset else 0)

@@ -5,8 +5,8 @@ ALL_ATTENTION_FUNCTIONS-style callable (experiments/llm/intra_token_attn.py:112-
 layers, then two 64-aligned-window layers, repeating, with dense attention for single-token decode
 steps because the patterns are prefill-only. This module offers the same callable with the prefill
 running on the B200 kernels: query/key/value arrive as (B, H, S, D) and are handed to the kernel as
-(B, S, H, D) views without copies. The decode step stays what it is in the reference - one dense SDPA
-call over the cache, outside the scope of the sparse kernels.
+(B, S, H, D) views without copies. The decode step is dense over the cache, as in the reference: on the
+library's decode kernel for bf16 caches with or without a padding mask, else one SDPA call.
 
     from transformers import AttentionInterface
     AttentionInterface.register("intra_b200", make_intra_attention())
@@ -17,7 +17,7 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
-from .interface import intra_llm_attn
+from .interface import decode_attn, intra_llm_attn
 
 NUM_GROUPS = 8          # intra_token_attn.py:22-24
 WINDOW_BACK = 512
@@ -41,6 +41,9 @@ def make_intra_attention(num_groups: int = NUM_GROUPS, back: int = WINDOW_BACK, 
     def intra_attention_forward(module, query, key, value, attention_mask=None, scaling=None, dropout=0.0,
                                 **kwargs):
         if query.shape[2] == 1:          # decode step: dense over the cache, as the reference does
+            out = decode_attn(query, key, value, attention_mask, scaling)
+            if out is not None:
+                return out, None
             rep = query.shape[1] // key.shape[1]
             k2 = key.repeat_interleave(rep, dim=1) if rep > 1 else key
             v2 = value.repeat_interleave(rep, dim=1) if rep > 1 else value

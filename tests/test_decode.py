@@ -1,0 +1,163 @@
+"""One-token decode of the transformers-style backend: the decode kernel against fp64 attention and against
+the SDPA call it stands in for, over the forms of cache and mask it takes; what it leaves to SDPA."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from intra_b200.interface import decode_attn
+from intra_b200.llm_backend import make_intra_attention
+
+
+def _inputs(B, H, Hkv, S, seed=0, layout="bhsd", device="cuda"):
+    g = torch.Generator().manual_seed(seed)
+    q = torch.randn(B, H, 1, 128, generator=g).to(torch.bfloat16).to(device)
+    shape = {"bhsd": (B, Hkv, S, 128), "bshd": (B, S, Hkv, 128), "sliced": (B, Hkv, S + 40, 128), "batch1": (1, Hkv, S, 128)}[layout]
+    k, v = (torch.randn(*shape, generator=g).to(torch.bfloat16).to(device) for _ in range(2))
+    if layout == "bshd":
+        k, v = k.transpose(1, 2), v.transpose(1, 2)
+    if layout == "sliced":                                   # a cache that is longer than what is filled
+        k[:, :, :3], v[:, :, :3], k[:, :, S + 3:], v[:, :, S + 3:] = (float("nan"),) * 4
+        k, v = k[:, :, 3:S + 3], v[:, :, 3:S + 3]
+    if layout == "batch1":
+        k, v = k.expand(B, -1, -1, -1), v.expand(B, -1, -1, -1)
+    return q, k, v
+
+
+def _mask(kind, B, S, device="cuda"):
+    g = torch.Generator().manual_seed(7)
+    if kind is None:
+        return None
+    if kind == "left-padded":
+        start = (S * 0.75 * torch.rand(B, 1, generator=g)).long()
+        start[0] = 0
+        m = torch.arange(S)[None, :] >= start
+    elif kind == "one-key":
+        m = torch.arange(S)[None, :].expand(B, S) == torch.randint(S, (B, 1), generator=g)
+    else:
+        m = torch.rand(1 if kind == "shared" else B, S, generator=g) < 0.3
+        m[:, -1] = True
+    if kind == "strided":
+        wide = torch.zeros(m.shape[0], 2 * S + 5, dtype=torch.bool)
+        wide[:, 5::2] = m
+        return wide.to(device)[:, None, None, 5::2]
+    if kind == "longer":                                     # cut to the cache's length by the backend's contract
+        m = torch.cat([m, torch.ones(m.shape[0], 9, dtype=torch.bool)], 1)
+    return m.to(device)[:, None, None, :]
+
+
+def _reference(q, k, v, mask, scale):
+    """fp64 result and sum_j p_j |v_j|, both (B, 1, H, 128)."""
+    rep = q.shape[1] // k.shape[1]
+    k, v = k.repeat_interleave(rep, 1).double(), v.repeat_interleave(rep, 1).double()
+    s = (q.double() @ k.transpose(-1, -2)) * scale
+    if mask is not None:
+        s = s.masked_fill(~mask[..., : k.shape[2]], float("-inf"))
+    p = s.softmax(-1)
+    return (p @ v).transpose(1, 2), (p @ v.abs()).transpose(1, 2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,Hkv,S,layout,mask", [
+    (1, 32, 8, 1, "bhsd", None), (1, 32, 8, 15, "bhsd", None), (1, 32, 8, 17, "bshd", None),       # ends of a 16-key block
+    (1, 4, 1, 63, "bhsd", "random"), (2, 32, 8, 64, "sliced", None), (3, 32, 8, 65, "batch1", "shared"),
+    (1, 32, 8, 1023, "bhsd", None), (1, 32, 8, 1024, "bhsd", None), (1, 32, 8, 3001, "bshd", None),   # clusters of 8 / 16
+    (1, 32, 8, 8191, "bhsd", None), (1, 4, 1, 40000, "sliced", None),                                 # several clusters
+    (16, 32, 8, 2100, "bhsd", "left-padded"), (20, 32, 32, 300, "bhsd", None), (300, 4, 1, 40, "bhsd", "one-key"),
+    (2, 9, 1, 500, "bhsd", "random"), (2, 36, 2, 77, "bhsd", "strided"), (1, 64, 2, 5000, "bshd", "longer"),   # 9, 18, 32 heads per KV head
+    (40, 16, 8, 2500, "bhsd", "random")])
+def test_decode_kernel_vs_fp64(B, H, Hkv, S, layout, mask):
+    q, k, v = _inputs(B, H, Hkv, S, layout=layout)
+    m = _mask(mask, B, S)
+    out = decode_attn(q, k, v, m, 0.1)
+    assert out is not None and out.shape == (B, 1, H, 128) and out.is_contiguous()
+    ref, spread = _reference(q, k, v, m, 0.1)
+    # half a bf16 ulp of the result (2^-8 |ref| covers it twice) + probabilities kept to 16 bits and fp32 sums:
+    # 2^-16 each, a factor four of margin
+    excess = (out.double() - ref).abs() - (2.0 ** -8 * ref.abs() + 2.0 ** -14 * spread)
+    assert float(excess.max()) <= 0
+    assert torch.equal(out, decode_attn(q, k, v, m, 0.1)), "two runs differ"
+    fn = make_intra_attention()
+    got, w = fn(None, q, k, v, m, scaling=0.1)
+    assert w is None and torch.equal(got, out)
+    rep = H // Hkv
+    sdpa = F.scaled_dot_product_attention(q, k.repeat_interleave(rep, 1), v.repeat_interleave(rep, 1),
+                                          attn_mask=None if m is None else m[..., :S], scale=0.1).transpose(1, 2)
+    worst = (out.double() - sdpa.double()).abs() - (2.0 ** -7 * ref.abs() + 2.0 ** -7 * spread)   # SDPA rounds P to bf16
+    assert float(worst.max()) <= 0
+
+
+@pytest.mark.gpu
+def test_decode_kernel_masked_keys_and_special_values():
+    q, k, v = _inputs(2, 8, 2, 200)
+    m = _mask("random", 2, 200)
+    clean = decode_attn(q, k, v, m)
+    k2, v2 = k.clone(), v.clone()
+    hidden = ~m[:, 0, 0, :]
+    k2[hidden[:, None].expand(2, 2, 200)] = float("nan")
+    v2[hidden[:, None].expand(2, 2, 200)] = float("inf")
+    assert torch.equal(decode_attn(q, k2, v2, m), clean), "a hidden key's row reached the result"
+    m0 = m.clone()
+    m0[1] = False                                              # a sequence that sees nothing
+    out = decode_attn(q, k, v, m0)
+    assert torch.equal(out[0], clean[0]) and not bool(out[1].any())
+    k3 = k.clone()
+    k3[0, :, 50] = float("nan")                                # a visible NaN reaches every head of its batch entry only
+    out = decode_attn(q, k3, v)
+    assert bool(out[0].isnan().all()) and bool(torch.isfinite(out[1]).all())
+    big = decode_attn(q * 50, k, v)                            # near one-hot rows
+    ref, spread = _reference(q * 50, k, v, None, 128 ** -0.5)
+    assert float(((big.double() - ref).abs() - (2.0 ** -8 * ref.abs() + 2.0 ** -11 * spread)).max()) <= 0   # fp32 scores of several hundred
+
+
+@pytest.mark.gpu
+def test_decode_kernel_under_capture_and_on_other_streams():
+    cases = [_inputs(1, 32, 8, 3001, seed=1), _inputs(1, 4, 1, 40000, seed=2)]
+    want = [decode_attn(*c) for c in cases]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got = [decode_attn(*c) for c in cases]
+    side.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = [decode_attn(*c) for c in cases]
+    for x in got:
+        x.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.gpu
+def test_calls_the_decode_kernel_leaves_to_sdpa():
+    q, k, v = _inputs(2, 8, 2, 64)
+    m = _mask("random", 2, 64)
+    fn = make_intra_attention()
+
+    def same_as_sdpa(q, k, v, m=None):
+        assert decode_attn(q, k, v, m) is None
+        rep = q.shape[1] // k.shape[1]
+        want = F.scaled_dot_product_attention(q, k.repeat_interleave(rep, 1), v.repeat_interleave(rep, 1), attn_mask=m).transpose(1, 2)
+        assert torch.equal(fn(None, q, k, v, m)[0], want)
+
+    same_as_sdpa(q.half(), k.half(), v.half())
+    same_as_sdpa(q[..., :64], k[..., :64], v[..., :64])
+    same_as_sdpa(q, k, v, torch.zeros(2, 1, 1, 64, device="cuda", dtype=torch.bfloat16))
+    same_as_sdpa(q, k, v, m.expand(2, 8, 1, 64))                               # a mask per head
+    same_as_sdpa(q, k.clone().requires_grad_(True), v)
+    wide = torch.randn(2, 2, 64, 132, device="cuda").bfloat16()[..., 2:130]     # rows that are not 16-byte aligned
+    same_as_sdpa(q, wide, v)
+    with torch.autocast("cuda", dtype=torch.float16):
+        assert decode_attn(q, k, v) is None and fn(None, q, k, v)[0].dtype == torch.float16
+    batched = torch.vmap(lambda a, b, c: fn(None, a, b, c)[0])(q[None], k[None], v[None])
+    assert float((batched[0].float() - decode_attn(q, k, v).float()).abs().max()) <= 1.6e-2
+
+
+def test_decode_on_the_cpu_is_sdpa():
+    q, k, v = _inputs(2, 8, 2, 30, device="cpu")
+    m = _mask("random", 2, 30, device="cpu")
+    assert decode_attn(q, k, v, m) is None
+    out, _ = make_intra_attention()(None, q, k, v, m)
+    want = F.scaled_dot_product_attention(q, k.repeat_interleave(4, 1), v.repeat_interleave(4, 1), attn_mask=m).transpose(1, 2)
+    assert torch.equal(out, want)
