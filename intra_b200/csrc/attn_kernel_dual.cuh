@@ -1,21 +1,21 @@
-// Persistent, ping-pong forward kernel: each CTA owns one SM and walks a static list of pair tiles
-// (intra_index.h): two 128-row query sub-tiles that share every K / V tile brought into shared
-// memory (or, for Gather-0, keep a K / V buffer each). While one sub-tile's softmax runs on the CUDA
-// cores, the tensor core works on the other's QK^T and PV, so the two pipes overlap inside one CTA.
+// Persistent, ping-pong forward kernel for shapes whose rows no TMA box describes (ragged Gather-1, odd image
+// widths, expanded tensors): 128 loader threads gather rows with cp.async. Everything else runs on
+// attn_kernel_rows.cuh. Each CTA owns one SM and walks a static list of pair tiles (intra_index.h): two
+// 128-row query sub-tiles that share every K / V tile brought into shared memory (or, for Gather-0, keep
+// a K / V buffer each). While one sub-tile's softmax runs on the CUDA cores, the tensor core works on the
+// other's QK^T and PV, so the two pipes overlap inside one CTA.
 //
 // Warp roles (N = softmax column split, 2 or 4):
 //   warps [0, 4N)      softmax / correction, all on one sub-tile at a time, alternating between the two:
 //                      warp w owns rows 32 (w % 4) .. +31 and score columns [(w / 4) * 128 / N, +128 / N)
-//                      (TMEM: S0 cols 0-127, S1 cols 128-255, O0 cols 256-383, O1 cols 384-511; P overlays S)
-//   warps [4N, 4N+4)   with TMA loads: epilogue (O of a finished item -> bf16 -> global while the softmax
-//                      warps are already on the next item); otherwise loaders: index maps + cp.async row
-//                      gathers whose completion the copies signal themselves
+//                      (TMEM: S0 cols 0-127, S1 cols 128-255, O0 cols 256-383, O1 cols 384-511; P overlays S);
+//                      at an item's end they store O
+//   warps [4N, 4N+4)   loaders: index maps + cp.async row gathers whose completion the copies signal themselves
 //   warp 4N+4          an elected thread issues tcgen05.mma in the order QK0(n) PV1(n-1) QK1(n) PV0(n),
 //                      carried across item boundaries so that the next item's first QK^T overlaps this
 //                      item's last softmax
-//   warp 4N+5          one thread issues the TMA loads: Q0, Q1 and a 2-stage ring each for K and V
 //   warp 4N+6          planner: decodes the CTA's items a few ahead into a ring in shared memory (key-tile
-//                      count, per-row token and key interval, TMA box coordinates) for all other roles
+//                      count, per-row token and key interval) for all other roles
 //
 // Items are dealt to CTAs heaviest first in boustrophedon order, which needs no counters in global
 // memory. Every wait is bounded; see attn_kernel.cuh for the abort protocol, which is the same.
@@ -29,9 +29,9 @@
 // Replaces, like attn_kernel.cuh, the reference's compute_attn_1rowblock_* kernels
 // (csrc/flash_attn/src/flash_fwd_kernel.h:3970-6158) for every pattern.
 #pragma once
+#include "attn_items.cuh"
 #include "attn_kernel.cuh"
 #include "softmax.cuh"
-#include "tma_maps.h"
 
 namespace intra {
 
@@ -66,175 +66,6 @@ constexpr int KV_STAGES = 2;
 constexpr int DUAL_SMEM_BYTES = (2 + 2 * KV_STAGES) * TILE_BYTES + 1024;   // Q0 Q1 | K ring | V ring
 constexpr int DUAL_TMEM_COLS = 512;
 
-struct DualParams {
-  FwdParams f;
-  int row_pairs;        // 0: sub-tiles are two heads of one KV group; 1: two row tiles of one head
-  int n_pair_tiles;     // pair tiles per (batch, head or head pair)
-  int heads_per_item;   // row_pairs ? H : H / 2  (number of items per pair tile and batch)
-  int n_items;          // n_pair_tiles * B * heads_per_item
-  int split_kv;         // the two sub-tiles keep their own key lists (Gather-0): K / V buffer s belongs to sub-tile s
-  int use_tma;          // tiles are fetched as TMA boxes (tma_maps.h) instead of cp.async row gathers; selects kTma
-  int wide_stores;      // every output row is 32-byte aligned: 256-bit global stores
-  TmaMaps maps;
-};
-
-// The tensor maps of one operand (Q, K or V).
-struct TmaOperand {
-  const CUtensorMap* main_map;
-  const CUtensorMap* text_map;
-  const CUtensorMap* aux_map;
-};
-
-// Fetch the 128 rows starting at `start` of tile `t` into the swizzled tile at `dst` (two boxes, one
-// per half of the head dim), completion counted on `bar`.
-__device__ __forceinline__ void tma_fetch_tile(const Problem& prob, const Tile& t, int start, bool text, int head,
-                                               int batch, const TmaOperand& op, uint32_t dst, uint64_t* bar) {
-  int c[5];
-  const int is_text = tma_box_coords(prob, t, start, text, head, batch, c);
-  const bool rank4 = tma_rank4(t, is_text);
-  // a Gather-0 problem's text tiles are image-Scatter tiles whose image keys come through the aux view
-  const CUtensorMap* m = is_text ? op.text_map : (prob.kind == KIND_IMG_GATHER0 ? op.aux_map : op.main_map);
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    if (rank4) ptx::tma_load_4d(dst + half * HALF_BYTES, m, bar, half * 64, c[1], c[2], c[3]);
-    else ptx::tma_load_5d(dst + half * HALF_BYTES, m, bar, half * 64, c[1], c[2], c[3], c[4]);
-  }
-}
-
-// Query rows of sub-tile `t` (TILE_BYTES in all).
-__device__ __forceinline__ void tma_fetch_q(const Problem& prob, const Tile& t, int head, int batch, const TmaOperand& op,
-                                            uint32_t dst, uint64_t* bar) {
-  if (t.kind == KIND_IMG_GATHER0) {                       // two 8x8 patches, 64 rows each
-#pragma unroll
-    for (int patch = 0; patch < 2; ++patch) {
-      const int pc = t.pcol + (patch == 1 && t.nq > PATCH * PATCH ? 1 : 0);   // no right patch: the left one again
-#pragma unroll
-      for (int half = 0; half < 2; ++half)
-        ptx::tma_load_5d(dst + half * HALF_BYTES + patch * (64 * 128), op.main_map, bar, half * 64, PATCH * pc,
-                         PATCH * t.prow, head, batch);
-    }
-    return;
-  }
-  int start; bool text;
-  tma_q_start(t, &start, &text);
-  tma_fetch_tile(prob, t, start, text, head, batch, op, dst, bar);
-}
-
-// Key tile n of key-slot map `kv` (TILE_BYTES).
-__device__ __forceinline__ void tma_fetch_kv(const Problem& prob, const Tile& kv, int n, int head, int batch,
-                                             const TmaOperand& op, uint32_t dst, uint64_t* bar) {
-  if (kv.kind == KIND_IMG_GATHER0) {
-    // slots: 16 window columns (2 tiles) | 512 text (4 tiles) | the right patch's extra columns (1 tile)
-    if (n >= 2 && n < 6) {
-#pragma unroll
-      for (int half = 0; half < 2; ++half)
-        ptx::tma_load_4d(dst + half * HALF_BYTES, op.text_map, bar, half * 64, TILE_N * (n - 2), head, batch);
-    } else {
-      const int wc0 = n < 2 ? 8 * n : WIN + 8 * (n - 6);
-#pragma unroll
-      for (int half = 0; half < 2; ++half)
-        ptx::tma_load_5d(dst + half * HALF_BYTES, op.main_map, bar, half * 64, kv.r0, kv.c0 + wc0, head, batch);
-    }
-    return;
-  }
-  int start; bool text;
-  tma_kv_start(kv, n, &start, &text);
-  tma_fetch_tile(prob, kv, start, text, head, batch, op, dst, bar);
-}
-
-struct DualItem {
-  PairTile pt;
-  int b, h0, h1, hk;
-};
-
-// Item number `seq` of this CTA: heaviest-first list dealt round by round, every other round reversed.
-INTRA_HD int dual_item_index(int seq, int cta, int n_cta) {
-  return seq * n_cta + ((seq & 1) ? (n_cta - 1 - cta) : cta);
-}
-
-INTRA_HD DualItem dual_decode(const DualParams& p, int item) {
-  DualItem it;
-  const int per_tile = p.f.B * p.heads_per_item;
-  const int idx = item / per_tile;
-  const int rem = item % per_tile;
-  it.b = rem / p.heads_per_item;
-  const int hh = rem % p.heads_per_item;
-  if (p.row_pairs) { it.h0 = it.h1 = hh; } else { it.h0 = 2 * hh; it.h1 = 2 * hh + 1; }
-  it.hk = it.h0 / (p.f.H / p.f.Hkv);
-  it.pt = make_pair(p.f.prob, p.row_pairs, idx);
-  return it;
-}
-
-// Normalise `ncols` (a multiple of 32) accumulator columns of this thread's TMEM lane by `inv` and store
-// them as bf16 to `dst` (this row's position in the output). `wide` selects 32-byte stores, which need
-// 32-byte aligned rows; tensor-memory loads are finished when the function returns.
-__device__ __forceinline__ void store_o_row(uint32_t o_addr, int ncols, float inv, __nv_bfloat16* dst, bool valid,
-                                            bool wide) {
-  for (int c = 0; c < ncols / 32; ++c) {
-    uint32_t o[32];
-    ptx::tmem_ld32(o_addr + c * 32, o);
-    ptx::tmem_wait_ld();
-    if (valid) {
-      uint32_t w[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        w[i] = ptx::pack_bf16(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
-      __nv_bfloat16* d = dst + c * 32;
-      if (wide) {
-        ptx::st_global_v8(d, w);
-        ptx::st_global_v8(d + 16, w + 8);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<uint4*>(d + i * 8) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-      }
-    }
-  }
-}
-
-// Box coordinates of an item's key tiles are affine in the tile number within at most two segments
-// (image kinds: the 512 text keys, then the image keys). The TMA thread works them out once per item
-// and afterwards only adds a constant per tile: it shares a scheduler with softmax warps, and every
-// instruction it spends per tile slows those down.
-struct KvSegment {
-  int c[5];          // coordinates of the segment's first tile (c[0] unused)
-  int d[5];          // increment per tile
-  int first;         // first tile of the segment
-  int text;          // 1: text map, 0: main / aux map
-  int rank4;
-};
-__device__ __forceinline__ void kv_segment(const Problem& prob, const Tile& kv, int first, int n_kv, int head, int batch,
-                                           KvSegment* sg) {
-  int start; bool text;
-  tma_kv_start(kv, first, &start, &text);
-  sg->first = first;
-  sg->text = tma_box_coords(prob, kv, start, text, head, batch, sg->c);
-  sg->rank4 = tma_rank4(kv, sg->text);
-  int c1[5];
-  if (first + 1 < n_kv) {
-    tma_kv_start(kv, first + 1, &start, &text);
-    tma_box_coords(prob, kv, start, text, head, batch, c1);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 5; ++i) c1[i] = sg->c[i];
-  }
-#pragma unroll
-  for (int i = 0; i < 5; ++i) sg->d[i] = c1[i] - sg->c[i];
-}
-__device__ __forceinline__ void tma_fetch_planned(const KvSegment& sg, int n, const CUtensorMap* m, uint32_t dst,
-                                                  uint64_t* bar) {
-  const int k = n - sg.first;
-  const int c1 = sg.c[1] + k * sg.d[1], c2 = sg.c[2] + k * sg.d[2], c3 = sg.c[3] + k * sg.d[3];
-  if (sg.rank4) {
-    ptx::tma_load_4d(dst, m, bar, 0, c1, c2, c3);
-    ptx::tma_load_4d(dst + HALF_BYTES, m, bar, 64, c1, c2, c3);
-  } else {
-    const int c4 = sg.c[4] + k * sg.d[4];
-    ptx::tma_load_5d(dst, m, bar, 0, c1, c2, c3, c4);
-    ptx::tma_load_5d(dst + HALF_BYTES, m, bar, 64, c1, c2, c3, c4);
-  }
-}
-
 // One entry of the CTA's item ring: everything any role needs to know about an item, worked out once
 // by the planner warp a few items ahead instead of by every warp at every item boundary (the index
 // arithmetic has divisions in it, and softmax warps have no issue slots to spare).
@@ -243,42 +74,15 @@ struct ItemSlot {
   int valid;                     // 0: end of this CTA's list
   int n_kv;                      // key tiles of the item (> 0)
   int b, h0, h1, hk;
-  // shared-key modes: what the TMA thread needs to request the tiles
-  int n_text;                    // tiles of the first key segment (== n_kv unless text + image keys)
-  int q0_text, q1_text, q0_rank4, q1_rank4;
-  KvSegment seg0, seg1;
-  int q0[5], q1[5];              // box coordinates of the two query sub-tiles
   PairTile pt;                   // for the cp.async loaders (key slots -> tokens)
   int token[2][TILE_M];          // per sub-tile and query row: token (-1: padding row) and its inclusive
   int lo[2][TILE_M];             // interval of key slots
   int hi[2][TILE_M];
 };
-__device__ __forceinline__ void plan_query(const Problem& prob, const Tile& t, int head, int batch, int c[5], int* is_text,
-                                           int* rank4) {
-  int start; bool text;
-  tma_q_start(t, &start, &text);
-  *is_text = tma_box_coords(prob, t, start, text, head, batch, c);
-  *rank4 = tma_rank4(t, *is_text);
-}
-// TMA box coordinates of an item's two query tiles and of its key tiles (shared-key modes), for the
-// thread that issues the loads.
-__device__ __forceinline__ void plan_slot_boxes(const DualParams& p, const DualItem& di, ItemSlot& sl) {
-  const int n_kv = di.pt.kv.n_kv_tiles;
-  const bool image_kind = di.pt.kv.kind == KIND_IMG_SCATTER;
-  const int n_text = image_kind && TEXT_LEN / TILE_N < n_kv ? TEXT_LEN / TILE_N : n_kv;
-  sl.n_text = n_text;
-  kv_segment(p.f.prob, di.pt.kv, 0, n_text, di.hk, di.b, &sl.seg0);
-  if (n_text < n_kv) kv_segment(p.f.prob, di.pt.kv, n_text, n_kv, di.hk, di.b, &sl.seg1);
-  // an absent sub-tile (odd tile count) is fed the other one's rows; its results are dropped
-  const Tile& t0 = di.pt.sub[0].n_kv_tiles > 0 ? di.pt.sub[0] : di.pt.sub[1];
-  const Tile& t1 = di.pt.sub[1].n_kv_tiles > 0 ? di.pt.sub[1] : di.pt.sub[0];
-  plan_query(p.f.prob, t0, di.h0, di.b, sl.q0, &sl.q0_text, &sl.q0_rank4);
-  plan_query(p.f.prob, t1, di.h1, di.b, sl.q1, &sl.q1_text, &sl.q1_rank4);
-}
 // Planner warp: fills ring slot after ring slot with the CTA's non-empty items, then one end marker.
 // slot_ready[r] completes once per fill of slot r; slot_free[r] once all consumers have let go of it.
 __device__ __forceinline__ void plan_items(const DualParams& p, ItemSlot* ring, uint64_t* slot_ready, uint64_t* slot_free,
-                                           int cta, int n_cta, int lane, bool plan_boxes, volatile int* abort_p) {
+                                           int cta, int n_cta, int lane, volatile int* abort_p) {
   int seq = 0;
   for (int i = 0;; ++i) {
     DualItem di;
@@ -286,7 +90,7 @@ __device__ __forceinline__ void plan_items(const DualParams& p, ItemSlot* ring, 
     for (;; ++seq) {
       const int item = dual_item_index(seq, cta, n_cta);
       if (item >= p.n_items) break;
-      di = dual_decode(p, item);
+      di = dual_decode(p, p.f.prob, item);
       if (di.pt.kv.n_kv_tiles > 0) { valid = true; ++seq; break; }
     }
     const int r = i % ITEM_RING;
@@ -315,7 +119,6 @@ __device__ __forceinline__ void plan_items(const DualParams& p, ItemSlot* ring, 
         sl.n_kv = n_kv;
         sl.b = di.b; sl.h0 = di.h0; sl.h1 = di.h1; sl.hk = di.hk;
         sl.pt = di.pt;
-        if (plan_boxes) plan_slot_boxes(p, di, sl);
       }
     }
     __syncwarp();
@@ -323,16 +126,6 @@ __device__ __forceinline__ void plan_items(const DualParams& p, ItemSlot* ring, 
     if (!valid) return;
   }
 }
-__device__ __forceinline__ void tma_fetch_box(const int c[5], int rank4, const CUtensorMap* m, uint32_t dst, uint64_t* bar) {
-  if (rank4) {
-    ptx::tma_load_4d(dst, m, bar, 0, c[1], c[2], c[3]);
-    ptx::tma_load_4d(dst + HALF_BYTES, m, bar, 64, c[1], c[2], c[3]);
-  } else {
-    ptx::tma_load_5d(dst, m, bar, 0, c[1], c[2], c[3], c[4]);
-    ptx::tma_load_5d(dst + HALF_BYTES, m, bar, 64, c[1], c[2], c[3], c[4]);
-  }
-}
-
 // Shared-memory layout and barriers the loaders of the split-K/V mode need.
 struct SplitLoaderCtx {
   uint32_t q_smem0, k_smem0, v_smem0;
@@ -346,60 +139,42 @@ struct SplitLoaderCtx {
 // buffer, refilled as soon as the MMA that read it has completed. Event driven: when QK0 of key tile
 // j is done (which, the pipe being in order, also means PV0 of tile j-1 is done) V0(j) and K0(j+1)
 // are requested; likewise for sub-tile 1, whose event also frees the Q buffers at an item's end.
-// kTma: one thread issues TMA boxes; otherwise all 128 loader threads gather rows with cp.async.
-template <bool kTma>
+// All 128 loader threads gather rows with cp.async.
 __device__ __forceinline__ void split_loader(const DualParams& p, const SplitLoaderCtx& cx, int lt) {
   const int chunk = lt & 15, rsub = lt >> 4;
-  const TmaOperand q_op = {&p.maps.q_main, &p.maps.q_text, &p.maps.q_main};
-  const TmaOperand k_op = {&p.maps.k_main, &p.maps.k_text, &p.maps.k_aux};
-  const TmaOperand v_op = {&p.maps.v_main, &p.maps.v_text, &p.maps.v_aux};
 
   auto fetch_q = [&](const ItemSlot& sl) {
-    if (kTma) {
-      ptx::mbar_arrive_expect_tx(cx.q_full, TILE_BYTES);
-      ptx::mbar_arrive_expect_tx(cx.q1_full, TILE_BYTES);
-      tma_fetch_q(p.f.prob, pair_kv_map(sl.pt, 1, 0), sl.h0, sl.b, q_op, cx.q_smem0, cx.q_full);
-      tma_fetch_q(p.f.prob, pair_kv_map(sl.pt, 1, 1), sl.h1, sl.b, q_op, cx.q_smem0 + TILE_BYTES, cx.q1_full);
-    } else {
 #pragma unroll 1
-      for (int sx = 0; sx < 2; ++sx) {
-        const __nv_bfloat16* qb = p.f.q + sl.b * p.f.qs.sb + (sx ? sl.h1 : sl.h0) * p.f.qs.sh + chunk * 8;
+    for (int sx = 0; sx < 2; ++sx) {
+      const __nv_bfloat16* qb = p.f.q + sl.b * p.f.qs.sb + (sx ? sl.h1 : sl.h0) * p.f.qs.sh + chunk * 8;
 #pragma unroll 4
-        for (int ps = 0; ps < TILE_M / 8; ++ps) {
-          const int row = ps * 8 + rsub;
-          const int token = sl.token[sx][row];
-          const void* src = token >= 0 ? static_cast<const void*>(qb + int64_t(token) * p.f.qs.ss) : static_cast<const void*>(p.f.q);
-          ptx::cp_async_16(cx.q_smem0 + sx * TILE_BYTES + tile_offset(row, chunk), src, token >= 0 ? 16u : 0u);
-        }
+      for (int ps = 0; ps < TILE_M / 8; ++ps) {
+        const int row = ps * 8 + rsub;
+        const int token = sl.token[sx][row];
+        const void* src = token >= 0 ? static_cast<const void*>(qb + int64_t(token) * p.f.qs.ss) : static_cast<const void*>(p.f.q);
+        ptx::cp_async_16(cx.q_smem0 + sx * TILE_BYTES + tile_offset(row, chunk), src, token >= 0 ? 16u : 0u);
       }
-      ptx::cp_async_mbar_arrive_noinc(cx.q_full);
-      ptx::cp_async_mbar_arrive_noinc(cx.q1_full);
     }
+    ptx::cp_async_mbar_arrive_noinc(cx.q_full);
+    ptx::cp_async_mbar_arrive_noinc(cx.q1_full);
   };
   auto fetch_kv = [&](bool is_v, int sx, const ItemSlot& sl, int n) {
     const Tile& map = pair_kv_map(sl.pt, 1, sx);
     const uint32_t dst = (is_v ? cx.v_smem0 : cx.k_smem0) + sx * TILE_BYTES;
     uint64_t* bar = is_v ? &cx.v_full[sx] : &cx.k_full[sx];
-    if (kTma) {
-      ptx::mbar_arrive_expect_tx(bar, TILE_BYTES);
-      tma_fetch_kv(p.f.prob, map, n, sl.hk, sl.b, is_v ? v_op : k_op, dst, bar);
-    } else {
-      const __nv_bfloat16* base = is_v ? p.f.v + sl.b * p.f.vs.sb + sl.hk * p.f.vs.sh + chunk * 8
-                                       : p.f.k + sl.b * p.f.ks.sb + sl.hk * p.f.ks.sh + chunk * 8;
-      const int64_t ss = is_v ? p.f.vs.ss : p.f.ks.ss;
+    const __nv_bfloat16* base = is_v ? p.f.v + sl.b * p.f.vs.sb + sl.hk * p.f.vs.sh + chunk * 8
+                                     : p.f.k + sl.b * p.f.ks.sb + sl.hk * p.f.ks.sh + chunk * 8;
+    const int64_t ss = is_v ? p.f.vs.ss : p.f.ks.ss;
 #pragma unroll 4
-      for (int ps = 0; ps < TILE_N / 8; ++ps) {
-        const int row = ps * 8 + rsub;
-        const int token = key_token(p.f.prob, map, n * TILE_N + row);
-        const void* src = token >= 0 ? static_cast<const void*>(base + int64_t(token) * ss) : static_cast<const void*>(p.f.k);
-        ptx::cp_async_16(dst + tile_offset(row, chunk), src, token >= 0 ? 16u : 0u);
-      }
-      ptx::cp_async_mbar_arrive_noinc(bar);
+    for (int ps = 0; ps < TILE_N / 8; ++ps) {
+      const int row = ps * 8 + rsub;
+      const int token = key_token(p.f.prob, map, n * TILE_N + row);
+      const void* src = token >= 0 ? static_cast<const void*>(base + int64_t(token) * ss) : static_cast<const void*>(p.f.k);
+      ptx::cp_async_16(dst + tile_offset(row, chunk), src, token >= 0 ? 16u : 0u);
     }
+    ptx::cp_async_mbar_arrive_noinc(bar);
   };
-  // one arrival per consumer warp; the TMA loader is a single thread
-  auto release = [&](int seq) {
-    if (kTma) { ptx::mbar_arrive(&cx.slot_free[seq % ITEM_RING]); return; }
+  auto release = [&](int seq) {                            // one arrival per consumer warp
     __syncwarp();
     if ((lt & 31) == 0) ptx::mbar_arrive(&cx.slot_free[seq % ITEM_RING]);
   };
@@ -414,7 +189,7 @@ __device__ __forceinline__ void split_loader(const DualParams& p, const SplitLoa
 
   int seq = 0, n = 0;                                      // the key tile being fed: tile n of item seq
   const ItemSlot* cur = acquire(0);
-  if (cur == nullptr) { if (!kTma) { ptx::cp_async_commit(); ptx::cp_async_wait<0>(); } return; }
+  if (cur == nullptr) { ptx::cp_async_commit(); ptx::cp_async_wait<0>(); return; }
   fetch_q(*cur);
   fetch_kv(false, 0, *cur, 0);
   fetch_kv(false, 1, *cur, 0);
@@ -434,10 +209,11 @@ __device__ __forceinline__ void split_loader(const DualParams& p, const SplitLoa
     cur = nxt;
     n = nn;
   }
-  if (!kTma) { ptx::cp_async_commit(); ptx::cp_async_wait<0>(); }
+  ptx::cp_async_commit();
+  ptx::cp_async_wait<0>();
 }
 
-template <int NSPLIT, bool kSplitKV, bool kTma>
+template <int NSPLIT, bool kSplitKV>
 __global__ void __launch_bounds__(DualCfg<NSPLIT>::THREADS, 1) intra_fwd_dual_kernel(const __grid_constant__ DualParams p) {
   using Cfg = DualCfg<NSPLIT>;
   constexpr int COLS = Cfg::COLS, SM_WARPS = Cfg::SM_WARPS, SM_THREADS = Cfg::SM_THREADS;
@@ -457,7 +233,6 @@ __global__ void __launch_bounds__(DualCfg<NSPLIT>::THREADS, 1) intra_fwd_dual_ke
   __shared__ int abort_flag;
   __shared__ float xch_max[2][NSPLIT][TILE_M];      // [phase parity][column part][row]: partial row maxima
   __shared__ float xch_sum[2][2][NSPLIT][TILE_M];   // [item parity][sub-tile][column part][row]: partial row sums
-  __shared__ float xch_m[2][2][TILE_M];             // [item parity][sub-tile][row]: the running maximum they refer to
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -490,7 +265,7 @@ __global__ void __launch_bounds__(DualCfg<NSPLIT>::THREADS, 1) intra_fwd_dual_ke
 
   if (tid == 0) {
     abort_flag = 0;
-    const uint32_t producers = kTma ? 1 : 128;       // one TMA-issuing thread, or every loader thread
+    const uint32_t producers = 128;                       // every loader thread
     ptx::mbar_init(q_full, producers);
     ptx::mbar_init(q1_full, producers);
     for (int j = 0; j < KV_STAGES; ++j) {
@@ -511,11 +286,10 @@ __global__ void __launch_bounds__(DualCfg<NSPLIT>::THREADS, 1) intra_fwd_dual_ke
     ptx::mbar_init(l_ready1, 4);
     ptx::mbar_init(pv0_done, 1);
     ptx::mbar_init(drain2, 1);
-    ptx::mbar_init(&o_free[0], (kTma || NSPLIT == 1) ? 128 : SM_THREADS);   // whoever runs the epilogue
-    ptx::mbar_init(&o_free[1], (kTma || NSPLIT == 1) ? 128 : SM_THREADS);
-    // ring consumers, one arrival per warp: softmax warps, the MMA warp, and either the four epilogue warps
-    // plus the TMA thread, or the four cp.async loader warps
-    const uint32_t consumers = SM_WARPS + (NSPLIT == 1 ? 2 : 1) + (kTma ? 5 : 4);
+    ptx::mbar_init(&o_free[0], NSPLIT == 1 ? 128 : SM_THREADS);
+    ptx::mbar_init(&o_free[1], NSPLIT == 1 ? 128 : SM_THREADS);
+    // ring consumers, one arrival per warp: softmax warps, the MMA warp(s), the four loader warps
+    const uint32_t consumers = SM_WARPS + (NSPLIT == 1 ? 2 : 1) + 4;
     for (int r = 0; r < ITEM_RING; ++r) {
       ptx::mbar_init(&slot_ready[r], 1);
       ptx::mbar_init(&slot_free[r], consumers);
@@ -674,23 +448,6 @@ __global__ void __launch_bounds__(DualCfg<NSPLIT>::THREADS, 1) intra_fwd_dual_ke
           if (lane == 0) ptx::mbar_arrive(&p_full[sx]);
         }
         if (!ok) break;
-        const int ipar = n_done & 1;
-        if (kTma) {                                       // the epilogue warps take it from here
-          // ... once they are done with this sub-tile of the item before: a set is not held back by the
-          // other set or by the PVs of an item of one key tile, so without this wait it could report two
-          // items before the epilogue warps have looked at the barrier once (and overwrite the sums of the
-          // item before the last, which they may still be reading).
-          if (n_done > 0) {
-            ok = ptx::mbar_wait(&o_free[sx], (n_done - 1) & 1, abort_p);
-            if (!ok) { if (*abort_p == 1) *abort_p = 19; break; }
-          }
-          xch_sum[ipar][sx][0][row] = l_run;
-          if (p.f.lse != nullptr) xch_m[ipar][sx][row] = m_run;
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(sx ? l_ready1 : l_ready);
-          ++n_done;
-          continue;
-        }
         ok = ptx::mbar_wait(&o_done[sx], n_done & 1, abort_p);       // last PV of this item
         if (!ok) { if (*abort_p == 1) *abort_p = 15 + sx; break; }
         ptx::tc_fence_after();
@@ -814,26 +571,8 @@ __global__ void __launch_bounds__(DualCfg<NSPLIT>::THREADS, 1) intra_fwd_dual_ke
 
       // ---- row sums: publish this half's share; whoever stores O adds the two halves ----------
       const int ipar = n_done & 1;
-      if (kTma && n_done > 0) {
-        // The epilogue warps must have taken the report of the item before (they have once they hand its
-        // first accumulator back) before the barrier may complete again. The order of the MMAs makes
-        // this wait return at once in practice; it turns that timing into a guarantee.
-        ok = ptx::mbar_wait(&o_free[0], (n_done - 1) & 1, abort_p);
-        if (!ok) { if (*abort_p == 1) *abort_p = 19; break; }
-      }
       xch_sum[ipar][0][half][row] = l_part[0];
       xch_sum[ipar][1][half][row] = l_part[1];
-      if (half == 0 && p.f.lse != nullptr) {              // every part of a row holds the same maximum
-        xch_m[ipar][0][row] = m_run[0];
-        xch_m[ipar][1][row] = m_run[1];
-      }
-      if (kTma) {
-        // the epilogue warps take it from here; go straight on to the next item
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(l_ready);
-        ++n_done;
-        continue;
-      }
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(xbar);
       ok = ptx::mbar_wait(xbar, ph & 1, abort_p);
@@ -869,49 +608,10 @@ __global__ void __launch_bounds__(DualCfg<NSPLIT>::THREADS, 1) intra_fwd_dual_ke
     bool ok = true;
     int n_done = 0;
 
-    if (kTma) {
-      // ---- epilogue warps: O of a finished item -> global, while the softmax warps are already on
-      //      the next item. Thread = query row (all 128 columns). ------------------------------------
-      const int row = tid & 127;
-      const uint32_t lane_addr = tmem + (uint32_t((warp & 3) * 32) << 16);
-      for (int seq = 0; ok; ++seq) {
-        INTRA_RING_ACQUIRE(sl, 53);
-        const int token[2] = {sl.token[0][row], sl.token[1][row]};
-        const int item_b = sl.b, item_h[2] = {sl.h0, sl.h1};
-        INTRA_RING_RELEASE_WARP();
-        const int ipar = n_done & 1;
-        if (NSPLIT > 1) {
-          ok = ptx::mbar_wait(l_ready, ipar, abort_p);
-          if (!ok) { if (*abort_p == 1) *abort_p = 41; break; }
-        }
-#pragma unroll
-        for (int sx = 0; sx < 2; ++sx) {
-          if (NSPLIT == 1) {                                       // each sub-tile's warp set reports for itself
-            ok = ptx::mbar_wait(sx ? l_ready1 : l_ready, ipar, abort_p);
-            if (!ok) { if (*abort_p == 1) *abort_p = 41; break; }
-          }
-          ok = ptx::mbar_wait(&o_done[sx], ipar, abort_p);         // last PV of this item
-          if (!ok) { if (*abort_p == 1) *abort_p = 42 + sx; break; }
-          ptx::tc_fence_after();
-          float l_tot = 0.f;
-#pragma unroll
-          for (int o = 0; o < NSPLIT; ++o) l_tot += xch_sum[ipar][sx][o][row];
-          const float inv = l_tot > 0.f ? 1.f / l_tot : 0.f;
-          const int h = item_h[sx];
-          const int tk = token[sx];
-          if (p.f.lse != nullptr && tk >= 0)
-            p.f.lse[(int64_t(item_b) * p.f.H + h) * p.f.prob.S + tk] = row_lse(xch_m[ipar][sx][row], l_tot, p.f.scale_log2);
-          __nv_bfloat16* dst = p.f.o + item_b * p.f.os.sb + int64_t(tk < 0 ? 0 : tk) * p.f.os.ss + h * p.f.os.sh;
-          store_o_row(lane_addr + 256 + sx * 128, 128, inv, dst, tk >= 0, p.wide_stores != 0);
-          ptx::tc_fence_before();
-          ptx::mbar_arrive(&o_free[sx]);                           // the next item's first PV may overwrite O
-        }
-        ++n_done;
-      }
-    } else if (kSplitKV) {
+    if (kSplitKV) {
       const SplitLoaderCtx cx = {q_smem0, k_smem0, v_smem0, q_full, q1_full, k_full, v_full, s0_full, s1_full,
                                  ring, slot_ready, slot_free, abort_p};
-      split_loader<false>(p, cx, lt);
+      split_loader(p, cx, lt);
     } else {
       // ---- cp.async row gathers by all 128 loader threads (ragged shapes) ------------------------
       const int chunk = lt & 15;                          // 16-byte chunk of the 256-byte row
@@ -983,74 +683,9 @@ __global__ void __launch_bounds__(DualCfg<NSPLIT>::THREADS, 1) intra_fwd_dual_ke
   } else {
     // ================================ MMA issue ==================================================
     ptx::setmaxnreg_dec<MMA_REGS>();
-    if (kSplitKV && warp == SM_WARPS + 5 && kTma && lane == 0) {
-      const SplitLoaderCtx cx = {q_smem0, k_smem0, v_smem0, q_full, q1_full, k_full, v_full, s0_full, s1_full,
-                                 ring, slot_ready, slot_free, abort_p};
-      split_loader<true>(p, cx, 0);
-    } else if (warp == SM_WARPS + 5 && kTma && lane == 0) {
-      // ---- one thread drives the TMA unit ------------------------------------------------------------
-      uint32_t kc = 0;                                    // K / V tiles requested so far (ring position)
-      bool ok = true;
-      int n_done = 0;
-      ptx::prefetch_tensormap(&p.maps.q_main);
-      ptx::prefetch_tensormap(&p.maps.k_main);
-      ptx::prefetch_tensormap(&p.maps.v_main);
-      const TmaOperand q_op = {&p.maps.q_main, &p.maps.q_text, &p.maps.q_main};
-      const TmaOperand k_op = {&p.maps.k_main, &p.maps.k_text, &p.maps.k_aux};
-      const TmaOperand v_op = {&p.maps.v_main, &p.maps.v_text, &p.maps.v_aux};
-      const CUtensorMap* k_main = p.f.prob.kind == KIND_IMG_GATHER0 ? k_op.aux_map : k_op.main_map;
-      const CUtensorMap* v_main = p.f.prob.kind == KIND_IMG_GATHER0 ? v_op.aux_map : v_op.main_map;
-      for (int seq = 0; ok; ++seq) {
-        INTRA_RING_ACQUIRE(sl, 55);
-        const int n_kv = sl.n_kv, n_text = sl.n_text;
-        for (int n = 0; n < n_kv && ok; ++n, ++kc) {
-          const int stage = kc % KV_STAGES;
-          const KvSegment& sg = n < n_text ? sl.seg0 : sl.seg1;
-          const CUtensorMap* kmap = sg.text ? k_op.text_map : k_main;
-          const CUtensorMap* vmap = sg.text ? v_op.text_map : v_main;
-          if (kc >= 2) {                                // K stage: QK1 of key tile kc-2
-            INTRA_WAIT_TILE_DONE(kc - 2, 22);
-            if (!ok) break;
-          }
-          ptx::mbar_arrive_expect_tx(&k_full[stage], TILE_BYTES);
-          tma_fetch_planned(sg, n, kmap, k_smem0 + stage * TILE_BYTES, &k_full[stage]);
-          if (n == 0) {
-            // The item's queries go in between its first K and V tiles, each as early as its buffer
-            // frees: Q0 after QK0 of the previous item's last key tile, Q1 after that tile's QK1.
-            if (n_done > 0) {
-              ok = ptx::mbar_wait(s0_full, (kc - 1) & 1, abort_p);
-              if (!ok) { if (*abort_p == 1) *abort_p = 21; break; }
-            }
-            ptx::mbar_arrive_expect_tx(q_full, TILE_BYTES);
-            tma_fetch_box(sl.q0, sl.q0_rank4, sl.q0_text ? q_op.text_map : q_op.main_map, q_smem0, q_full);
-          }
-          if (NSPLIT == 1) {                            // Q1: QK1 of the previous item's last key tile; V stage: PV1 of kc-2
-            if (n == 0 && n_done > 0) {
-              INTRA_WAIT_TILE_DONE(kc - 1, 23);
-              if (!ok) break;
-            }
-            if (kc >= 2) {
-              INTRA_WAIT_V_STAGE(kc, 26);
-              if (!ok) break;
-            }
-          } else if (kc >= 2 || (n == 0 && n_done > 0)) {   // V stage: PV1 of key tile kc-2, issued before QK1 of kc-1
-            INTRA_WAIT_TILE_DONE(kc - 1, 23);
-            if (!ok) break;
-          }
-          if (n == 0) {
-            ptx::mbar_arrive_expect_tx(q1_full, TILE_BYTES);
-            tma_fetch_box(sl.q1, sl.q1_rank4, sl.q1_text ? q_op.text_map : q_op.main_map, q_smem0 + TILE_BYTES, q1_full);
-          }
-          ptx::mbar_arrive_expect_tx(&v_full[stage], TILE_BYTES);
-          tma_fetch_planned(sg, n, vmap, v_smem0 + stage * TILE_BYTES, &v_full[stage]);
-        }
-        if (!ok) break;
-        ptx::mbar_arrive(&slot_free[seq % ITEM_RING]);
-        ++n_done;
-      }
-    } else if (warp == SM_WARPS + 6) {
+    if (warp == SM_WARPS + 6) {
       // ---- planner: keeps the item ring filled -------------------------------------------------------
-      plan_items(p, ring, slot_ready, slot_free, cta, n_cta, lane, kTma && !kSplitKV, abort_p);
+      plan_items(p, ring, slot_ready, slot_free, cta, n_cta, lane, abort_p);
     }
     if ((warp == SM_WARPS + 4 || warp == SM_WARPS + 7) && NSPLIT == 1) {
       // ---- row-owner form: two issuing warps, so that neither kind of product waits for the other's

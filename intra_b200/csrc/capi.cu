@@ -15,6 +15,7 @@
 
 #include "attn_kernel.cuh"
 #include "attn_kernel_dual.cuh"
+#include "attn_kernel_rows.cuh"
 #include "decode_kernel.cuh"
 #include "gather_kernel.cuh"
 #include "selftest.cuh"
@@ -36,14 +37,11 @@ DeviceState g_dev[MAX_DEVICES];
 
 // Test hook (intra_b200_test_force_path): overrides of the launcher's own choice of kernel variant.
 std::atomic<int> g_force_no_tma{0};      // 1: cp.async row gathers even where TMA boxes would do
-// Items with at least this many key tiles on average go to the row-owner form of the kernel
-// (attn_kernel_dual.cuh); below it the 4-way column split is faster (measured: equal at 8.5 key tiles
-// per item, 18-22 % behind on window patterns with their 5 key tiles, most of them masked at an edge).
-#ifndef INTRA_ROW_OWNER_MIN_TILES
-#define INTRA_ROW_OWNER_MIN_TILES 8
-#endif
-constexpr int ROW_OWNER_MIN_TILES = INTRA_ROW_OWNER_MIN_TILES;
-std::atomic<int> g_force_split{0};       // 1 (row-owner form), 2 or 4: softmax column split; 0: the launcher decides
+// Row-gather kernel (attn_kernel_dual.cuh): items with at least this many key tiles on average go to its
+// row-owner form; below it the 4-way column split is faster (measured: equal at 8.5 key tiles per item, 18-22 %
+// behind on window patterns with their 5 key tiles). The TMA kernel has one form for all lengths.
+constexpr int ROW_OWNER_MIN_TILES = 8;
+std::atomic<int> g_force_split{0};       // 1 (row-owner form), 2 or 4: its softmax column split; 0: the launcher decides
 
 int cuda_fail(cudaError_t e) {
   g_last_cuda_error = static_cast<int>(e);
@@ -70,16 +68,16 @@ cudaError_t opt_in_smem(K kernel, int bytes) {
 }
 cudaError_t set_kernel_attributes() {
   cudaError_t e = opt_in_smem(umma_selftest_kernel, SELFTEST_SMEM_BYTES);
-  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<1, false, true>, DUAL_SMEM_BYTES);
-  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<1, false, false>, DUAL_SMEM_BYTES);
-  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<2, false, true>, DUAL_SMEM_BYTES);
-  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<2, false, false>, DUAL_SMEM_BYTES);
-  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<4, false, true>, DUAL_SMEM_BYTES);
-  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<4, false, false>, DUAL_SMEM_BYTES);
-  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<2, true, true>, DUAL_SMEM_BYTES);
-  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<2, true, false>, DUAL_SMEM_BYTES);
-  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<4, true, true>, DUAL_SMEM_BYTES);
-  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<4, true, false>, DUAL_SMEM_BYTES);
+  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_rows_kernel<KIND_LLM_SCATTER>, ROWS_SMEM_BYTES);
+  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_rows_kernel<KIND_LLM_GATHER1>, ROWS_SMEM_BYTES);
+  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_rows_kernel<KIND_LLM_WINDOW>, ROWS_SMEM_BYTES);
+  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_rows_kernel<KIND_IMG_SCATTER>, ROWS_SMEM_BYTES);
+  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_rows_kernel<KIND_IMG_GATHER0>, ROWS_SMEM_BYTES);
+  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<1, false>, DUAL_SMEM_BYTES);
+  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<2, false>, DUAL_SMEM_BYTES);
+  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<4, false>, DUAL_SMEM_BYTES);
+  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<2, true>, DUAL_SMEM_BYTES);
+  if (e == cudaSuccess) e = opt_in_smem(intra_fwd_dual_kernel<4, true>, DUAL_SMEM_BYTES);
   return e;
 }
 
@@ -160,9 +158,12 @@ bool encode_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* di
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The views of tma_maps.h for one (batch, token, head, 128) tensor with `heads` heads.
-bool build_maps(const Problem& p, const __nv_bfloat16* ptr, const TensorView& tv, int heads, int B, bool is_query,
-                CUtensorMap* main_map, CUtensorMap* text_map, CUtensorMap* aux_map) {
+// The views of tma_maps.h for one (batch, token, head, 128) tensor with `heads` heads; operand 0 q, 1 k, 2 v.
+bool build_maps(const Problem& p, const __nv_bfloat16* ptr, const TensorView& tv, int heads, int B, int operand, TmaMaps* maps) {
+  CUtensorMap* const main_map = &maps->view[VIEW_MAIN][operand];
+  CUtensorMap* const text_map = &maps->view[VIEW_TEXT][operand];
+  CUtensorMap* const aux_map = &maps->view[VIEW_AUX][operand];
+  const bool is_query = operand == 0;
   const cuuint64_t ss = cuuint64_t(tv.ss) * 2, sh = cuuint64_t(tv.sh) * 2, sb = cuuint64_t(tv.sb) * 2;
   if (tv.ss <= 0 || tv.sh <= 0 || tv.sb <= 0) return false;
   const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
@@ -186,10 +187,10 @@ bool build_maps(const Problem& p, const __nv_bfloat16* ptr, const TensorView& tv
       return encode_map(main_map, ptr, 5, dims, str, box, ones);
     }
     case KIND_LLM_WINDOW: {
-      const cuuint64_t dims[4] = {128, cuuint64_t(p.S), cuuint64_t(heads), cuuint64_t(B)};
-      const cuuint64_t str[3] = {ss, sh, sb};
-      const cuuint32_t box[4] = {64, 128, 1, 1};
-      return encode_map(main_map, ptr, 4, dims, str, box, ones);
+      const cuuint64_t dims[5] = {128, cuuint64_t(p.S), 1, cuuint64_t(heads), cuuint64_t(B)};
+      const cuuint64_t str[4] = {ss, ss, sh, sb};
+      const cuuint32_t box[5] = {64, 128, 1, 1, 1};
+      return encode_map(main_map, ptr, 5, dims, str, box, ones);
     }
     case KIND_IMG_SCATTER: {
       const cuuint64_t dims[5] = {128, cuuint64_t(p.W), cuuint64_t(p.W), cuuint64_t(heads), cuuint64_t(B)};
@@ -197,10 +198,10 @@ bool build_maps(const Problem& p, const __nv_bfloat16* ptr, const TensorView& tv
       const cuuint32_t box[5] = {64, cuuint32_t(p.W), cuuint32_t(2 * (TILE_M / (p.W / 4))), 1, 1};
       const cuuint32_t estr[5] = {1, 4, 2, 1, 1};
       if (!encode_map(main_map, ptr + int64_t(TEXT_LEN) * tv.ss, 5, dims, str, box, estr)) return false;
-      const cuuint64_t tdims[4] = {128, TEXT_LEN, cuuint64_t(heads), cuuint64_t(B)};
-      const cuuint64_t tstr[3] = {ss, sh, sb};
-      const cuuint32_t tbox[4] = {64, 128, 1, 1};
-      return encode_map(text_map, ptr, 4, tdims, tstr, tbox, ones);
+      const cuuint64_t tdims[5] = {128, TEXT_LEN, 1, cuuint64_t(heads), cuuint64_t(B)};
+      const cuuint64_t tstr[4] = {ss, ss, sh, sb};
+      const cuuint32_t tbox[5] = {64, 128, 1, 1, 1};
+      return encode_map(text_map, ptr, 5, tdims, tstr, tbox, ones);
     }
     case KIND_IMG_GATHER0: {
       // patch-pair tiles: keys as 16-row x 8-column boxes (row index fastest), queries as 8x8 patches
@@ -220,10 +221,10 @@ bool build_maps(const Problem& p, const __nv_bfloat16* ptr, const TensorView& tv
         const cuuint32_t aestr[5] = {1, 4, 2, 1, 1};
         if (!encode_map(aux_map, img, 5, dims, astr, abox, aestr)) return false;
       }
-      const cuuint64_t tdims[4] = {128, TEXT_LEN, cuuint64_t(heads), cuuint64_t(B)};
-      const cuuint64_t tstr[3] = {ss, sh, sb};
-      const cuuint32_t tbox[4] = {64, 128, 1, 1};
-      return encode_map(text_map, ptr, 4, tdims, tstr, tbox, ones);
+      const cuuint64_t tdims[5] = {128, TEXT_LEN, 1, cuuint64_t(heads), cuuint64_t(B)};
+      const cuuint64_t tstr[4] = {ss, ss, sh, sb};
+      const cuuint32_t tbox[5] = {64, 128, 1, 1, 1};
+      return encode_map(text_map, ptr, 5, tdims, tstr, tbox, ones);
     }
     default:
       return false;
@@ -284,10 +285,10 @@ int check_args(const void* q, const void* k, const void* v, void* out, int B, in
   return INTRA_OK;
 }
 
-// How the launcher splits a problem into the persistent kernel's items, and which kernel variant it
+// How the launcher splits a problem into the persistent kernels' items, and which kernel variant it
 // picks (the counterpart of the reference's MASK_SWITCH / launch templates,
 // csrc/flash_attn/src/flash_fwd_launch_template.h:401-565, :720-776).
-// Softmax arrangement (attn_kernel_dual.cuh) for a problem: 4 = 4-way column split (short items),
+// Softmax arrangement of the row-gather kernel (attn_kernel_dual.cuh) for a problem: 4 = 4-way column split (short items),
 // 1 = row-owner form (long items that share their key tiles), 2 = 2-way split (long items with split
 // key lists). Host arithmetic only.
 int pick_form(const Problem& prob, int row_pairs, int split_kv) {
@@ -312,12 +313,14 @@ int plan_launch(const FwdParams& p, DualParams* d, int* split) {
   const int64_t items = int64_t(d->n_pair_tiles) * p.B * d->heads_per_item;
   if (items <= 0 || items > 0x7fffffffLL) return INTRA_ERR_UNSUPPORTED;
   d->n_items = static_cast<int>(items);
+  d->by_tile = fast_div(p.B * d->heads_per_item);
+  d->by_heads = fast_div(d->heads_per_item);
+  d->by_rep = fast_div(p.H / p.Hkv);
   d->wide_stores = (reinterpret_cast<uintptr_t>(p.o) % 32 == 0 && p.os.sb % 16 == 0 && p.os.ss % 16 == 0 && p.os.sh % 16 == 0) ? 1 : 0;
   d->use_tma = !g_force_no_tma.load() && tma_supported(p.prob) &&
-               build_maps(p.prob, p.q, p.qs, p.H, p.B, true, &d->maps.q_main, &d->maps.q_text, &d->maps.k_aux) &&
-               build_maps(p.prob, p.k, p.ks, p.Hkv, p.B, false, &d->maps.k_main, &d->maps.k_text, &d->maps.k_aux) &&
-               build_maps(p.prob, p.v, p.vs, p.Hkv, p.B, false, &d->maps.v_main, &d->maps.v_text, &d->maps.v_aux);
-  *split = pick_form(p.prob, d->row_pairs, d->split_kv);
+               build_maps(p.prob, p.q, p.qs, p.H, p.B, 0, &d->maps) && build_maps(p.prob, p.k, p.ks, p.Hkv, p.B, 1, &d->maps) &&
+               build_maps(p.prob, p.v, p.vs, p.Hkv, p.B, 2, &d->maps);
+  *split = d->use_tma ? 0 : pick_form(p.prob, d->row_pairs, d->split_kv);
   return INTRA_OK;
 }
 
@@ -345,16 +348,24 @@ int launch_fwd(const void* q, const void* k, const void* v, void* out, int B, in
   int rc = plan_launch(p, &d, &split);
   if (rc != INTRA_OK) return rc;
   const int grid = d.n_items < sm_count ? d.n_items : sm_count;     // persistent: one CTA per SM
-#define INTRA_LAUNCH_DUAL(N, SPLIT) \
-  do { \
-    if (d.use_tma) intra_fwd_dual_kernel<N, SPLIT, true><<<grid, DualCfg<N>::THREADS, DUAL_SMEM_BYTES, st>>>(d); \
-    else intra_fwd_dual_kernel<N, SPLIT, false><<<grid, DualCfg<N>::THREADS, DUAL_SMEM_BYTES, st>>>(d); \
-  } while (0)
-  if (split == 4 && d.split_kv) INTRA_LAUNCH_DUAL(4, true);
+#define INTRA_LAUNCH_ROWS(KIND) \
+  case KIND: intra_fwd_rows_kernel<KIND><<<grid, RowsCfg::THREADS, ROWS_SMEM_BYTES, st>>>(d); break
+#define INTRA_LAUNCH_DUAL(N, SPLIT) intra_fwd_dual_kernel<N, SPLIT><<<grid, DualCfg<N>::THREADS, DUAL_SMEM_BYTES, st>>>(d)
+  if (d.use_tma) {
+    switch (prob.kind) {
+      INTRA_LAUNCH_ROWS(KIND_LLM_SCATTER);
+      INTRA_LAUNCH_ROWS(KIND_LLM_GATHER1);
+      INTRA_LAUNCH_ROWS(KIND_LLM_WINDOW);
+      INTRA_LAUNCH_ROWS(KIND_IMG_SCATTER);
+      INTRA_LAUNCH_ROWS(KIND_IMG_GATHER0);
+      default: return INTRA_ERR_UNSUPPORTED;
+    }
+  } else if (split == 4 && d.split_kv) INTRA_LAUNCH_DUAL(4, true);
   else if (split == 4) INTRA_LAUNCH_DUAL(4, false);
   else if (d.split_kv) INTRA_LAUNCH_DUAL(2, true);
   else if (split == 2) INTRA_LAUNCH_DUAL(2, false);
   else INTRA_LAUNCH_DUAL(1, false);
+#undef INTRA_LAUNCH_ROWS
 #undef INTRA_LAUNCH_DUAL
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e);
@@ -766,7 +777,7 @@ int intra_b200_test_tma_rows(const void* q, const void* k, const void* v, int B,
 
   // what should arrive: -9 = any row will do (padding rows, slots no query attends)
   for (int item = 0; item < d.n_items; ++item) {
-    const DualItem di = dual_decode(d, item);
+    const DualItem di = dual_decode(d, prob, item);
     for (int sx = 0; sx < 2; ++sx) {
       int32_t* qw = q_want + (size_t(item) * 2 + sx) * TILE_M;
       int32_t* kw = k_want + (size_t(item) * 2 + sx) * mk * TILE_N;
@@ -791,8 +802,17 @@ int intra_b200_test_tma_rows(const void* q, const void* k, const void* v, int B,
   }
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   const int smem = TILE_BYTES + 1024;
-  if (d.split_kv) tma_rows_selftest_kernel<true><<<d.n_items, 128, smem, st>>>(d, q_got_dev, k_got_dev, v_got_dev, mk);
-  else tma_rows_selftest_kernel<false><<<d.n_items, 128, smem, st>>>(d, q_got_dev, k_got_dev, v_got_dev, mk);
+#define INTRA_ROWS_TEST(KIND) \
+  case KIND: tma_rows_selftest_kernel<KIND><<<d.n_items, 128, smem, st>>>(d, q_got_dev, k_got_dev, v_got_dev, mk); break
+  switch (prob.kind) {
+    INTRA_ROWS_TEST(KIND_LLM_SCATTER);
+    INTRA_ROWS_TEST(KIND_LLM_GATHER1);
+    INTRA_ROWS_TEST(KIND_LLM_WINDOW);
+    INTRA_ROWS_TEST(KIND_IMG_SCATTER);
+    INTRA_ROWS_TEST(KIND_IMG_GATHER0);
+    default: return INTRA_ERR_UNSUPPORTED;
+  }
+#undef INTRA_ROWS_TEST
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? INTRA_OK : cuda_fail(e);
 }

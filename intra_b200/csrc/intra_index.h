@@ -46,6 +46,24 @@ INTRA_HD int ceil_div(int a, int b) { return (a + b - 1) / b; }
 INTRA_HD int imin(int a, int b) { return a < b ? a : b; }
 INTRA_HD int imax(int a, int b) { return a > b ? a : b; }
 
+// Division of 0 <= n < 2^31 by a constant known on the host: one wide multiply and a shift. The planner warp of
+// the attention kernel divides a dozen times per item; the general division's code (some 25 instructions each)
+// counts there, because the kernel's code competes for the SM's instruction cache.
+struct FastDiv {
+  uint32_t d, mul;
+  int shift;
+};
+INTRA_HD FastDiv fast_div(int d) {
+  FastDiv f;
+  f.d = uint32_t(d);
+  int log2 = 0;
+  while (log2 < 31 && (uint64_t(1) << log2) < uint64_t(d)) ++log2;
+  f.shift = 31 + log2;
+  f.mul = uint32_t(((uint64_t(1) << f.shift) + uint64_t(d) - 1) / uint64_t(d));   // <= 2^32 - 1: d > 2^(log2 - 1)
+  return f;
+}
+INTRA_HD int fdiv(int n, const FastDiv& f) { return int((uint64_t(uint32_t(n)) * f.mul) >> f.shift); }
+
 struct Problem {
   int kind;
   int S;        // tokens per sequence
@@ -56,20 +74,21 @@ struct Problem {
   int n_img;    // image kinds: image tokens per group = W*W/8
   int pairs_per_row;  // gather0: patch pairs per patch row
   int n_longer;       // scatter: the first S % G groups have one token more than the others
+  int n_base, n_rem;  // group lengths: S / G (scatter); G * (S / G^2) and S % G^2 (gather1)
+  FastDiv by_G, by_quads, by_pairs, by_mp;   // G, W / 4, pairs_per_row, row pairs per image-Scatter group
 };
 
 // Length of group g's packed token list for the two grouped LLM patterns.
-INTRA_HD int llm_group_len(int kind, int S, int G, int g) {
-  if (kind == KIND_LLM_SCATTER) return S / G + (g < S % G ? 1 : 0);
-  const int span = G * G;                  // one segment of every group
-  const int rem = S % span;
-  return (S / span) * G + imin(imax(rem - g * G, 0), G);
+INTRA_HD int llm_group_len(const Problem& p, int kind, int g) {
+  if (kind == KIND_LLM_SCATTER) return p.n_base + (g < p.n_longer ? 1 : 0);
+  return p.n_base + imin(imax(p.n_rem - g * p.G, 0), p.G);
 }
 
 // Token id of packed index t in group g.
-INTRA_HD int llm_group_token(int kind, int G, int g, int t) {
-  if (kind == KIND_LLM_SCATTER) return t * G + g;
-  return (t / G) * G * G + g * G + t % G;
+INTRA_HD int llm_group_token(const Problem& p, int kind, int g, int t) {
+  if (kind == KIND_LLM_SCATTER) return t * p.G + g;
+  const int seg = fdiv(t, p.by_G);
+  return seg * p.G * p.G + g * p.G + (t - seg * p.G);
 }
 
 // First row / column of the 16-wide Gather-0 window of patch index x (of np patches per edge):
@@ -85,15 +104,23 @@ INTRA_HD int make_problem(int kind, int S, int G, int W, Problem* out) {
   Problem p;
   p.kind = kind; p.S = S; p.G = G; p.W = W;
   p.n_tiles = 0; p.tiles_m = 0; p.n_img = 0; p.pairs_per_row = 0; p.n_longer = 0;
+  p.n_base = 0; p.n_rem = 0;
   if (S <= 0) return -1;
+  p.by_G = fast_div(G > 0 ? G : 1);
+  p.by_quads = p.by_pairs = p.by_mp = fast_div(1);
   switch (kind) {
     case KIND_LLM_SCATTER:
     case KIND_LLM_GATHER1: {
       if (G <= 0 || G > S) return -1;
-      int nmax = 0;
-      for (int g = 0; g < G; ++g) nmax = imax(nmax, llm_group_len(kind, S, G, g));
-      if (kind == KIND_LLM_SCATTER) p.n_longer = S % G;
-      p.tiles_m = ceil_div(nmax, TILE_M);
+      if (kind == KIND_LLM_SCATTER) {
+        p.n_base = S / G;
+        p.n_longer = S % G;
+      } else {
+        const int64_t span = int64_t(G) * G;     // one segment of every group
+        p.n_base = int(S / span) * G;
+        p.n_rem = int(S % span);
+      }
+      p.tiles_m = ceil_div(llm_group_len(p, kind, 0), TILE_M);     // no group is longer than the first
       p.n_tiles = p.tiles_m * G;
       break;
     }
@@ -107,10 +134,14 @@ INTRA_HD int make_problem(int kind, int S, int G, int W, Problem* out) {
       p.G = IMG_GROUPS;
       p.n_img = W * W / IMG_GROUPS;
       p.tiles_m = 1 + ceil_div(p.n_img, TILE_M);
+      p.by_G = fast_div(IMG_GROUPS);
+      p.by_quads = fast_div(W / 4);
+      p.by_mp = fast_div(ceil_div(p.tiles_m, 2));
       if (kind == KIND_IMG_SCATTER) {
         p.n_tiles = p.tiles_m * IMG_GROUPS;
       } else {
         p.pairs_per_row = ceil_div(W / PATCH, 2);
+        p.by_pairs = fast_div(p.pairs_per_row);
         p.n_tiles = IMG_GROUPS + (W / PATCH) * p.pairs_per_row;
       }
       break;
@@ -145,10 +176,10 @@ INTRA_HD Tile make_tile(const Problem& p, int idx) {
   switch (p.kind) {
     case KIND_LLM_SCATTER:
     case KIND_LLM_GATHER1: {
-      const int m = p.tiles_m - 1 - idx / p.G;
-      t.g = idx % p.G;
-      t.t0 = m * TILE_M;
-      t.nq = llm_group_len(p.kind, p.S, p.G, t.g);
+      const int level = fdiv(idx, p.by_G);
+      t.g = idx - level * p.G;
+      t.t0 = (p.tiles_m - 1 - level) * TILE_M;
+      t.nq = llm_group_len(p, p.kind, t.g);
       if (t.t0 < t.nq) {
         t.nk = imin(t.t0 + TILE_M, t.nq);     // causal: no key beyond the tile's last query
         t.n_kv_tiles = ceil_div(t.nk, TILE_N);
@@ -184,8 +215,8 @@ INTRA_HD Tile make_tile(const Problem& p, int idx) {
       }
       const int pp = idx - IMG_GROUPS;
       const int np = p.W / PATCH;
-      t.prow = pp / p.pairs_per_row;
-      t.pcol = 2 * (pp % p.pairs_per_row);
+      t.prow = fdiv(pp, p.by_pairs);
+      t.pcol = 2 * (pp - t.prow * p.pairs_per_row);
       t.r0 = gather0_start(t.prow, np);
       t.c0 = gather0_start(t.pcol, np);
       const bool has_right = t.pcol + 1 < np;
@@ -201,10 +232,10 @@ INTRA_HD Tile make_tile(const Problem& p, int idx) {
 }
 
 // Token id of image-scatter group member u (u-th image token of group g in raster order).
-INTRA_HD int img_scatter_token(int W, int g, int u) {
-  const int quads = W / 4;                       // group members per grid row
+INTRA_HD int img_scatter_token(const Problem& p, int g, int u) {
+  const int row = fdiv(u, p.by_quads);           // W / 4 group members per grid row
   const int a = g / 4, b = g % 4;                // (row parity, column mod 4)
-  return TEXT_LEN + (u / quads) * 2 * W + (u % quads) * 4 + a * W + b;
+  return TEXT_LEN + row * 2 * p.W + (u - row * (p.W / 4)) * 4 + a * p.W + b;
 }
 
 // Query row r of tile t: token id (or -1 if the row is padding) and the inclusive key-slot
@@ -216,7 +247,7 @@ INTRA_HD void q_row(const Problem& p, const Tile& t, int r, int* token, int* lo,
     case KIND_LLM_SCATTER:
     case KIND_LLM_GATHER1: {
       const int q = t.t0 + r;
-      if (q < t.nq) { *token = llm_group_token(t.kind, p.G, t.g, q); *hi = q; }
+      if (q < t.nq) { *token = llm_group_token(p, t.kind, t.g, q); *hi = q; }
       break;
     }
     case KIND_LLM_WINDOW: {
@@ -231,7 +262,7 @@ INTRA_HD void q_row(const Problem& p, const Tile& t, int r, int* token, int* lo,
     case KIND_IMG_SCATTER: {
       const int u = t.t0 + r;
       if (t.is_text) { if (r < TEXT_CHUNK) *token = t.g * TEXT_CHUNK + r; }
-      else if (u < t.nq) *token = img_scatter_token(p.W, t.g, u);
+      else if (u < t.nq) *token = img_scatter_token(p, t.g, u);
       break;
     }
     case KIND_IMG_GATHER0: {
@@ -258,11 +289,11 @@ INTRA_HD int key_token(const Problem& p, const Tile& t, int u) {
   switch (t.kind) {
     case KIND_LLM_SCATTER:
     case KIND_LLM_GATHER1:
-      return llm_group_token(t.kind, p.G, t.g, u);
+      return llm_group_token(p, t.kind, t.g, u);
     case KIND_LLM_WINDOW:
       return t.kbase + u;
     case KIND_IMG_SCATTER:
-      return u < TEXT_LEN ? u : img_scatter_token(p.W, t.g, u - TEXT_LEN);
+      return u < TEXT_LEN ? u : img_scatter_token(p, t.g, u - TEXT_LEN);
     case KIND_IMG_GATHER0: {
       int v;
       if (u < WIN * WIN) v = u;
@@ -316,7 +347,7 @@ INTRA_HD PairTile make_pair(const Problem& p, int row_pairs, int idx) {
   switch (p.kind) {
     case KIND_LLM_SCATTER:
     case KIND_LLM_GATHER1: {
-      const int g = idx % p.G, mp = idx / p.G;
+      const int mp = fdiv(idx, p.by_G), g = idx - mp * p.G;
       idx_second = (2 * mp) * p.G + g;
       if (2 * mp + 1 < p.tiles_m) idx_first = (2 * mp + 1) * p.G + g;
       break;
@@ -330,7 +361,7 @@ INTRA_HD PairTile make_pair(const Problem& p, int row_pairs, int idx) {
       // moment are the row pairs of a few (head, group) key sets that stay in L2, instead of one row
       // pair of every group, which re-reads every key set from DRAM once per row pair.
       const int n_mp = ceil_div(p.tiles_m, 2);
-      const int g = idx / n_mp, mp = idx % n_mp;
+      const int g = fdiv(idx, p.by_mp), mp = idx - g * n_mp;
       idx_first = (2 * mp) * IMG_GROUPS + g;
       if (2 * mp + 1 < p.tiles_m) idx_second = (2 * mp + 1) * IMG_GROUPS + g;
       break;

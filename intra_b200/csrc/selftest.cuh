@@ -5,7 +5,7 @@
 // rows arrived; and a kernel whose wait is never satisfied, to exercise the abort protocol.
 #pragma once
 #include "attn_kernel.cuh"
-#include "attn_kernel_dual.cuh"
+#include "attn_kernel_rows.cuh"
 
 namespace intra {
 
@@ -135,37 +135,30 @@ __device__ __forceinline__ int decode_row_token(const uint8_t* tile, int row, in
   return tok[0] == tok[1] ? tok[0] : -2;
 }
 
-template <bool kSplitKV>
+template <int KIND>
 __global__ void __launch_bounds__(128, 1)
 tma_rows_selftest_kernel(const __grid_constant__ DualParams p, int* q_out, int* k_out, int* v_out, int max_kv) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar;
   __shared__ int abort_flag;
-  __shared__ ItemSlot sl;
+  __shared__ RowSlot sl;
   const int tid = threadIdx.x;
   const int item = blockIdx.x;
   const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint8_t* tile = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
-  const DualItem di = dual_decode(p, item);
-  const int n_kv = di.pt.kv.n_kv_tiles;
-  if (n_kv == 0) return;                                   // CTA-uniform
+  const uint32_t bar_at = ptx::smem_u32(&bar);
   if (tid == 0) {
     abort_flag = 0;
     ptx::mbar_init(&bar, 1);
     ptx::fence_mbar_init();
-    sl.pt = di.pt;
-    sl.b = di.b; sl.h0 = di.h0; sl.h1 = di.h1; sl.hk = di.hk;
-    if (!kSplitKV) plan_slot_boxes(p, di, sl);
+    plan_row_slot<KIND>(p, item, sl);
   }
   __syncthreads();
-  const TmaOperand q_op = {&p.maps.q_main, &p.maps.q_text, &p.maps.q_main};
-  const TmaOperand k_op = {&p.maps.k_main, &p.maps.k_text, &p.maps.k_aux};
-  const TmaOperand v_op = {&p.maps.v_main, &p.maps.v_text, &p.maps.v_aux};
-  const CUtensorMap* k_main = p.f.prob.kind == KIND_IMG_GATHER0 ? k_op.aux_map : k_op.main_map;
-  const CUtensorMap* v_main = p.f.prob.kind == KIND_IMG_GATHER0 ? v_op.aux_map : v_op.main_map;
+  const int n_kv = sl.n_kv;
+  if (n_kv == 0) return;                                   // CTA-uniform
   uint32_t phase = 0;
   bool ok = true;
-  // fetch(): thread 0 has issued one tile's loads onto `bar`; everyone waits for them and reads a row.
+  // collect(): thread 0 has issued one tile's loads onto `bar`; everyone waits for them and reads a row.
   auto collect = [&](int* dst, int head, int tensor_id) {
     ok = ok && ptx::mbar_wait(&bar, phase & 1, &abort_flag, 1000);
     ++phase;
@@ -173,28 +166,14 @@ tma_rows_selftest_kernel(const __grid_constant__ DualParams p, int* q_out, int* 
     __syncthreads();                                       // the buffer is reused by the next fetch
   };
   for (int sx = 0; sx < 2; ++sx) {
-    if (tid == 0 && abort_flag == 0) {
-      ptx::mbar_arrive_expect_tx(&bar, TILE_BYTES);
-      if (kSplitKV) tma_fetch_q(p.f.prob, pair_kv_map(sl.pt, 1, sx), sx ? sl.h1 : sl.h0, sl.b, q_op, smem_base, &bar);
-      else if (sx == 0) tma_fetch_box(sl.q0, sl.q0_rank4, sl.q0_text ? q_op.text_map : q_op.main_map, smem_base, &bar);
-      else tma_fetch_box(sl.q1, sl.q1_rank4, sl.q1_text ? q_op.text_map : q_op.main_map, smem_base, &bar);
-    }
-    collect(q_out + (size_t(item) * 2 + sx) * TILE_M, sx ? sl.h1 : sl.h0, 0);
+    if (tid == 0 && abort_flag == 0) fetch_q_tile(p.maps, sl.q[sx], sl.h[sx], sl.b, smem_base, bar_at);
+    collect(q_out + (size_t(item) * 2 + sx) * TILE_M, sl.h[sx], 0);
   }
   for (int is_v = 0; is_v < 2; ++is_v) {
     int* out = is_v ? v_out : k_out;
-    for (int sx = 0; sx < (kSplitKV ? 2 : 1); ++sx) {
+    for (int sx = 0; sx < (KIND == KIND_IMG_GATHER0 ? 2 : 1); ++sx) {
       for (int n = 0; n < n_kv; ++n) {
-        if (tid == 0 && abort_flag == 0) {
-          ptx::mbar_arrive_expect_tx(&bar, TILE_BYTES);
-          if (kSplitKV) {
-            tma_fetch_kv(p.f.prob, pair_kv_map(sl.pt, 1, sx), n, sl.hk, sl.b, is_v ? v_op : k_op, smem_base, &bar);
-          } else {
-            const KvSegment& sg = n < sl.n_text ? sl.seg0 : sl.seg1;
-            const CUtensorMap* m = is_v ? (sg.text ? v_op.text_map : v_main) : (sg.text ? k_op.text_map : k_main);
-            tma_fetch_planned(sg, n, m, smem_base, &bar);
-          }
-        }
+        if (tid == 0 && abort_flag == 0) fetch_kv_tile(p.maps, 1 + is_v, sl.kv[sx], n, sl.hk, sl.b, smem_base, bar_at);
         collect(out + ((size_t(item) * 2 + sx) * max_kv + n) * TILE_N, sl.hk, 1 + is_v);
       }
     }

@@ -5,18 +5,21 @@
 //
 //   Scatter                      dims (d, g, t, head, batch)       box (64, 1, 128)      token = t*G + g
 //             S % G = r > 0: groups 0..r-1 are one token longer, so there are two such views with exact extents:
-//             the "text" map holds groups 0..r-1 with S/G + 1 tokens each, the main map groups r..G-1 (base at
+//             the "text" view holds groups 0..r-1 with S/G + 1 tokens each, the main view groups r..G-1 (base at
 //             token r) with S/G. Nothing beyond token S-1 is ever read; the box rows past a group's end are
 //             zero-filled. Before, these shapes took the row gathers, whose 128 threads could not keep two K / V
 //             stages full: Scatter G=8, S=12345, 32/8 heads 423 us, 229 us as boxes (one launch, one B200).
 //   Gather-1 (S % G^2 == 0, G|128) dims (d, w, seg, head, batch)   box (64, G, 128/G)    token = seg*G^2 + w, w = g*G + j
-//   window                       dims (d, token, head, batch)      box (64, 128)
+//   window                       dims (d, token, 1, head, batch)   box (64, 128)
 //   image Scatter, image part    dims (d, c, r, head, batch), traversal strides (1, 4, 2), base at token 512
 //                                box (64, W, 2*128/(W/4)): every 4th column from c = b, every 2nd row from r = a
-//                text part       dims (d, token, head, batch), 512 tokens, box (64, 128)
+//                text part       dims (d, token, 1, head, batch), 512 tokens, box (64, 128)
 //   Gather-0 patch pairs  keys   dims (d, r, c, head, batch), box (64, 16, 8): 8 window columns, 16 rows each
 //                        queries dims (d, c, r, head, batch), box (64, 8, 8): one 8x8 patch, two boxes per tile
-//            text chunks         as image Scatter (the "aux" map) + the text map
+//            text chunks         as image Scatter (the "aux" view) + the text view
+//
+// All views have five dimensions (one of extent 1 where four would do), so that the requesting thread has a single
+// form of load to issue.
 //
 // Shapes outside these conditions (ragged Gather-1, odd widths) use the cp.async gathers.
 // This replaces the per-thread address arithmetic of the reference's loaders
@@ -28,17 +31,20 @@
 
 namespace intra {
 
+enum ViewId : int {
+  VIEW_MAIN = 0,    // the pattern's strided view
+  VIEW_TEXT = 1,    // image kinds: the 512 text tokens; ragged Scatter: its longer groups
+  VIEW_AUX = 2      // Gather-0: image-Scatter view for the keys of its text tiles
+};
 struct alignas(64) TmaMaps {
-  CUtensorMap q_main, k_main, v_main;   // the pattern's strided view
-  CUtensorMap q_text, k_text, v_text;   // image kinds: the 512 text tokens; ragged Scatter: its longer groups
-  CUtensorMap k_aux, v_aux;             // Gather-0: image-Scatter view for the keys of its text tiles
+  CUtensorMap view[3][3];   // [ViewId][query, key, value]
 };
 
 // Can the problem's tiles be fetched as TMA boxes?
 INTRA_HD bool tma_supported(const Problem& p) {
   switch (p.kind) {
     case KIND_LLM_SCATTER: return true;
-    case KIND_LLM_GATHER1: return p.S % (p.G * p.G) == 0 && TILE_M % p.G == 0 && p.G * p.G <= 65536;
+    case KIND_LLM_GATHER1: return TILE_M % p.G == 0 && p.S % (p.G * p.G) == 0;
     case KIND_LLM_WINDOW: return true;
     case KIND_IMG_SCATTER:
     case KIND_IMG_GATHER0:
@@ -47,51 +53,93 @@ INTRA_HD bool tma_supported(const Problem& p) {
   }
 }
 
-// Box coordinates (innermost first; c[0] is filled by the caller with 0 or 64) of the 128 rows that
-// start at `start` in the tile's own numbering: packed index for Scatter / Gather-1 and image
-// Scatter image rows, token id for the window and for text rows. Returns 1 if the text map is meant
-// (for Scatter: the view of the longer groups).
-INTRA_HD int tma_box_coords(const Problem& p, const Tile& t, int start, bool text, int head, int batch, int c[5]) {
-  c[0] = 0; c[1] = 0; c[2] = 0; c[3] = 0; c[4] = 0;
+// Box coordinates c1, c2 (c0 is the half of the head dim, c3 the head, c4 the batch) and view of a query tile.
+struct QPlan {
+  int which;         // ViewId
+  int c1, c2;
+  int patches;       // Gather-0: the tile is two 64-row boxes, one per 8x8 patch, the second at (c1b, c2)
+  int c1b;
+};
+// The same of an item's key tiles: tiles [text_lo, text_hi) are the 512 text tokens, the others
+// (numbered without them) lie at (c1, c2) + i * (s1, s2) of view `which`.
+struct KvPlan {
+  int which;
+  int text_lo, text_hi;
+  int c1, c2, s1, s2;
+};
+
+// Grid rows of the image a tile of an image-Scatter group spans.
+INTRA_HD int img_tile_rows(const Problem& p) { return 2 * fdiv(TILE_M, p.by_quads); }
+
+// View and first coordinates of the rows of a Scatter / Gather-1 / window / image-Scatter tile's numbering,
+// starting at its beginning.
+INTRA_HD void tma_origin(const Problem& p, const Tile& t, int* which, int* c1, int* c2) {
+  *which = VIEW_MAIN; *c1 = 0; *c2 = 0;
   switch (t.kind) {
     case KIND_LLM_SCATTER:
-      c[1] = t.g < p.n_longer ? t.g : t.g - p.n_longer;
-      c[2] = start; c[3] = head; c[4] = batch;
-      return t.g < p.n_longer;
-    case KIND_LLM_GATHER1:
-      c[1] = t.g * p.G; c[2] = start / p.G; c[3] = head; c[4] = batch;
-      return 0;
-    case KIND_LLM_WINDOW:
-      c[1] = start; c[2] = head; c[3] = batch;
-      return 0;
+      *which = t.g < p.n_longer ? VIEW_TEXT : VIEW_MAIN;
+      *c1 = t.g < p.n_longer ? t.g : t.g - p.n_longer;
+      break;
+    case KIND_LLM_GATHER1: *c1 = t.g * p.G; break;
+    case KIND_LLM_WINDOW: *c1 = t.kbase; break;
     case KIND_IMG_SCATTER:
-      if (text) { c[1] = start; c[2] = head; c[3] = batch; return 1; }
-      c[1] = t.g % 4; c[2] = t.g / 4 + 2 * (start / (p.W / 4)); c[3] = head; c[4] = batch;
-      return 0;
+      *which = p.kind == KIND_IMG_GATHER0 ? VIEW_AUX : VIEW_MAIN;
+      *c1 = t.g % 4; *c2 = t.g / 4;
+      break;
+    default: break;
+  }
+}
+
+// Query sub-tile `t`.
+INTRA_HD QPlan plan_q(const Problem& p, const Tile& t) {
+  QPlan q;
+  q.patches = 0; q.c1b = 0;
+  if (t.kind == KIND_IMG_GATHER0) {
+    q.which = VIEW_MAIN;
+    q.c1 = PATCH * t.pcol; q.c2 = PATCH * t.prow;
+    q.patches = 1;
+    q.c1b = PATCH * (t.pcol + (t.nq > PATCH * PATCH ? 1 : 0));    // no right patch: the left one again
+    return q;
+  }
+  tma_origin(p, t, &q.which, &q.c1, &q.c2);
+  switch (t.kind) {
+    case KIND_LLM_SCATTER: q.c2 = t.t0; break;
+    case KIND_LLM_GATHER1: q.c2 = fdiv(t.t0, p.by_G); break;
+    case KIND_LLM_WINDOW: q.c1 = t.t0; break;
     default:
-      return 0;
+      if (t.is_text) { q.which = VIEW_TEXT; q.c1 = t.g * TEXT_CHUNK; q.c2 = 0; }
+      else q.c2 += (t.t0 / TILE_M) * img_tile_rows(p);
+      break;
   }
+  return q;
 }
 
-// Is the box of a tile of this kind described by a rank-4 view (d, token, head, batch)?
-INTRA_HD int tma_rank4(const Tile& t, int is_text) {
-  return t.kind == KIND_LLM_WINDOW || (is_text && t.kind == KIND_IMG_SCATTER);
-}
-
-// Query sub-tile `t`: where its 128 rows start and whether they are text rows.
-INTRA_HD void tma_q_start(const Tile& t, int* start, bool* text) {
-  *text = false;
-  *start = t.t0;
-  if (t.kind == KIND_IMG_SCATTER && t.is_text) { *text = true; *start = t.g * TEXT_CHUNK; }
-}
-// Key tile n of key-slot map `kv`.
-INTRA_HD void tma_kv_start(const Tile& kv, int n, int* start, bool* text) {
-  *text = false;
-  *start = n * TILE_N;
-  if (kv.kind == KIND_LLM_WINDOW) *start += kv.kbase;
-  if (kv.kind == KIND_IMG_SCATTER) {
-    if (*start < TEXT_LEN) *text = true; else *start -= TEXT_LEN;
+// Key tiles of key-slot map `t`.
+INTRA_HD KvPlan plan_kv(const Problem& p, const Tile& t) {
+  KvPlan k;
+  k.text_lo = k.text_hi = 0; k.s1 = 0; k.s2 = 0;
+  if (t.kind == KIND_IMG_GATHER0) {
+    // slots: 16 window columns (2 tiles) | 512 text (4 tiles) | the right patch's extra columns (1 tile)
+    k.which = VIEW_MAIN;
+    k.text_lo = WIN * WIN / TILE_N; k.text_hi = k.text_lo + TEXT_LEN / TILE_N;
+    k.c1 = t.r0; k.c2 = t.c0; k.s2 = TILE_N / WIN;
+    return k;
   }
+  tma_origin(p, t, &k.which, &k.c1, &k.c2);
+  switch (t.kind) {
+    case KIND_LLM_SCATTER: k.s2 = TILE_N; break;
+    case KIND_LLM_GATHER1: k.s2 = fdiv(TILE_N, p.by_G); break;
+    case KIND_LLM_WINDOW: k.s1 = TILE_N; break;
+    default: k.text_hi = TEXT_LEN / TILE_N; k.s2 = img_tile_rows(p); break;
+  }
+  return k;
+}
+INTRA_HD void kv_box(const KvPlan& k, int n, int* which, int* c1, int* c2) {
+  const bool text = n >= k.text_lo && n < k.text_hi;
+  const int i = n < k.text_lo ? n : n - (k.text_hi - k.text_lo);
+  *which = text ? int(VIEW_TEXT) : k.which;
+  *c1 = text ? (n - k.text_lo) * TILE_N : k.c1 + i * k.s1;
+  *c2 = text ? 0 : k.c2 + i * k.s2;
 }
 
 }  // namespace intra
