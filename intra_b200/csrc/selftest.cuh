@@ -151,7 +151,8 @@ tma_rows_selftest_kernel(const __grid_constant__ DualParams p, int* q_out, int* 
     abort_flag = 0;
     ptx::mbar_init(&bar, 1);
     ptx::fence_mbar_init();
-    plan_row_slot<KIND>(p, item, sl);
+    const Problem pr = kind_problem<KIND>(p);
+    fill_row_slot<KIND>(pr, dual_decode(p, pr, item), sl);
   }
   __syncthreads();
   const int n_kv = sl.n_kv;
