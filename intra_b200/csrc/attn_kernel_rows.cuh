@@ -53,7 +53,8 @@ struct RowsCfg {
   static_assert(256 * SM_REGS + 128 * (EP_REGS + MMA_REGS) <= 65536,
                 "register budgets exceed what the CTA was launched with: setmaxnreg.inc would never return");
 };
-constexpr int ROWS_SMEM_BYTES = 6 * TILE_BYTES + 1024;     // Q0 Q1 | K0 K1 | V0 V1
+constexpr int OUT_STAGE = OUT_ROWS * 128;                  // bytes an epilogue warp stages: 64 columns of its rows
+constexpr int ROWS_SMEM_BYTES = 6 * TILE_BYTES + 4 * OUT_STAGE + 1024;     // Q0 Q1 | K0 K1 | V0 V1 | output staging
 
 // One item of the CTA's list.
 struct RowSlot {
@@ -167,6 +168,7 @@ template <int KIND>
 __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(const __grid_constant__ DualParams p) {
   using Cfg = RowsCfg;
   constexpr bool SPLIT = KIND == KIND_IMG_GATHER0;         // sub-tile s has K / V buffer s to itself
+  constexpr bool IMAGE = KIND == KIND_IMG_SCATTER || KIND == KIND_IMG_GATHER0;
   enum : int {
     Q_FULL = 0, K_FULL = 2, V_FULL = 4, S_FULL = 6, PV_DONE = 10, P_FULL = 14, S_TAKEN = 16, O_DONE = 18, O_FREE = 20,
     L_READY = 22, BATCH_READY = 24, BATCH_FREE = 26, DRAIN = 28, N_BARS = 30
@@ -348,23 +350,66 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
     ROWS_ITEMS(53)
 #pragma unroll 1
       for (int sx = 0; sx < 2; ++sx) {
-        int token, lo, hi;
-        slot_row<KIND>(p.f.prob, sl, sx, row, &token, &lo, &hi);
         const int b = sl.b, h = sl.h[sx];
         ok = ROWS_WAIT(L_READY + sx, seq, 41) && ROWS_WAIT(O_DONE + sx, seq, 43 + sx);
         if (!ok) break;
         ptx::tc_fence_after();
         const float l = row_sum[seq & 1][sx][row];
         const float inv = l > 0.f ? 1.f / l : 0.f;
+        const uint32_t o_addr = lane_addr + 256 + sx * 128;
+        int token = -1, lo, hi;
+        if (IMAGE || p.f.lse != nullptr) slot_row<KIND>(p.f.prob, sl, sx, row, &token, &lo, &hi);
         if (p.f.lse != nullptr && token >= 0)
           p.f.lse[(int64_t(b) * p.f.H + h) * p.f.prob.S + token] = row_lse(row_max[seq & 1][sx][row], l, p.f.scale_log2);
-        __nv_bfloat16* const dst = p.f.o + b * p.f.os.sb + int64_t(token < 0 ? 0 : token) * p.f.os.ss + h * p.f.os.sh;
-        store_o_row(lane_addr + 256 + sx * 128, HEAD_DIM, inv, dst, token >= 0, p.wide_stores != 0);
+        if (IMAGE) {
+          __nv_bfloat16* const dst = p.f.o + b * p.f.os.sb + int64_t(token < 0 ? 0 : token) * p.f.os.ss + h * p.f.os.sh;
+          store_o_row(o_addr, HEAD_DIM, inv, dst, token >= 0, p.wide_stores != 0);
+        } else {
+          // A warp's 32 rows leave as two bulk stores of 64 columns each through its staging buffer (128-byte swizzle).
+          // Stored by their threads, 32 bytes to 32 lines per instruction, they would hold up the sets' barrier
+          // traffic behind them: GPU time of Scatter at S = 4096 30.2 -> 28.7 us, window at 16384 155.4 -> 151.2.
+          // The image patterns' strided views have no such boxes; their rows are stored by their threads.
+          const int w = warp & 3;
+          int c1 = sl.q[sx].c1, c2 = sl.q[sx].c2;          // the query tile's place, this warp's rows on
+          if (KIND == KIND_LLM_SCATTER) c2 += OUT_ROWS * w;
+          if (KIND == KIND_LLM_WINDOW) c1 += OUT_ROWS * w;
+          if (KIND == KIND_LLM_GATHER1) { const int seg = fdiv(OUT_ROWS * w, p.f.prob.by_G); c1 += OUT_ROWS * w - seg * p.f.prob.G; c2 += seg; }
+          const bool wanted = sl.sub[sx].n_kv_tiles > 0 && sl.sub[sx].t0 + OUT_ROWS * w < sl.sub[sx].nq;
+          const CUtensorMap* const m = &p.maps.view[sl.q[sx].which][3];
+          const uint32_t stage = v_smem + 2 * TILE_BYTES + w * OUT_STAGE;
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t o[32];
+            ptx::tmem_ld32(o_addr + c * 32, o);
+            if ((c & 1) == 0) {                            // the staging buffer's last store has read it
+              if (lane == 0) ptx::bulk_wait_read();
+              __syncwarp();
+            }
+            ptx::tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint32_t x[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                x[e] = ptx::pack_bf16(__uint_as_float(o[8 * i + 2 * e]) * inv, __uint_as_float(o[8 * i + 2 * e + 1]) * inv);
+              ptx::st_shared_v4(stage + lane * 128 + ((((c & 1) * 4 + i) ^ (lane & 7)) << 4), x[0], x[1], x[2], x[3]);
+            }
+            if (c & 1) {
+              ptx::fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0 && wanted) {
+                ptx::tma_store_5d(m, stage, (c >> 1) * 64, c1, c2, h, b);
+                ptx::bulk_commit();
+              }
+            }
+          }
+        }
         ptx::tc_fence_before();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive_at(bar(O_FREE + sx));        // the next item's first PV may overwrite O
       }
     ROWS_ITEMS_END(0xffffffffu)
+    if (!IMAGE && lane == 0) ptx::bulk_wait_read();        // the staging buffers live until their stores have read them
   } else {
     ptx::setmaxnreg_dec<Cfg::MMA_REGS>();
     if (warp == 14) {

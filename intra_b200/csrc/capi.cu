@@ -158,12 +158,14 @@ bool encode_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* di
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The views of tma_maps.h for one (batch, token, head, 128) tensor with `heads` heads; operand 0 q, 1 k, 2 v.
+// The views of tma_maps.h for one (batch, token, head, 128) tensor with `heads` heads; operand 0 q, 1 k, 2 v, 3 the
+// output, whose boxes have 32 rows and which only the language-model patterns store through views.
 bool build_maps(const Problem& p, const __nv_bfloat16* ptr, const TensorView& tv, int heads, int B, int operand, TmaMaps* maps) {
   CUtensorMap* const main_map = &maps->view[VIEW_MAIN][operand];
   CUtensorMap* const text_map = &maps->view[VIEW_TEXT][operand];
   CUtensorMap* const aux_map = &maps->view[VIEW_AUX][operand];
   const bool is_query = operand == 0;
+  const int rows = operand == 3 ? OUT_ROWS : TILE_M;
   const cuuint64_t ss = cuuint64_t(tv.ss) * 2, sh = cuuint64_t(tv.sh) * 2, sb = cuuint64_t(tv.sb) * 2;
   if (tv.ss <= 0 || tv.sh <= 0 || tv.sb <= 0) return false;
   const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
@@ -172,7 +174,7 @@ bool build_maps(const Problem& p, const __nv_bfloat16* ptr, const TensorView& tv
       const int longer = p.n_longer;      // groups 0..longer-1 have one token more: a view of their own
       cuuint64_t dims[5] = {128, cuuint64_t(p.G - longer), cuuint64_t(p.S / p.G), cuuint64_t(heads), cuuint64_t(B)};
       const cuuint64_t str[4] = {ss, ss * p.G, sh, sb};
-      const cuuint32_t box[5] = {64, 1, 128, 1, 1};
+      const cuuint32_t box[5] = {64, 1, cuuint32_t(rows), 1, 1};
       if (!encode_map(main_map, ptr + int64_t(longer) * tv.ss, 5, dims, str, box, ones)) return false;
       if (longer == 0) return true;
       dims[1] = longer;
@@ -183,13 +185,14 @@ bool build_maps(const Problem& p, const __nv_bfloat16* ptr, const TensorView& tv
       const cuuint64_t span = cuuint64_t(p.G) * p.G;
       const cuuint64_t dims[5] = {128, span, cuuint64_t(p.S) / span, cuuint64_t(heads), cuuint64_t(B)};
       const cuuint64_t str[4] = {ss, ss * span, sh, sb};
-      const cuuint32_t box[5] = {64, cuuint32_t(p.G), cuuint32_t(TILE_M / p.G), 1, 1};
+      const int in_segment = imin(p.G, rows);
+      const cuuint32_t box[5] = {64, cuuint32_t(in_segment), cuuint32_t(rows / in_segment), 1, 1};
       return encode_map(main_map, ptr, 5, dims, str, box, ones);
     }
     case KIND_LLM_WINDOW: {
       const cuuint64_t dims[5] = {128, cuuint64_t(p.S), 1, cuuint64_t(heads), cuuint64_t(B)};
       const cuuint64_t str[4] = {ss, ss, sh, sb};
-      const cuuint32_t box[5] = {64, 128, 1, 1, 1};
+      const cuuint32_t box[5] = {64, cuuint32_t(rows), 1, 1, 1};
       return encode_map(main_map, ptr, 5, dims, str, box, ones);
     }
     case KIND_IMG_SCATTER: {
@@ -319,7 +322,9 @@ int plan_launch(const FwdParams& p, DualParams* d, int* split) {
   d->wide_stores = (reinterpret_cast<uintptr_t>(p.o) % 32 == 0 && p.os.sb % 16 == 0 && p.os.ss % 16 == 0 && p.os.sh % 16 == 0) ? 1 : 0;
   d->use_tma = !g_force_no_tma.load() && tma_supported(p.prob) &&
                build_maps(p.prob, p.q, p.qs, p.H, p.B, 0, &d->maps) && build_maps(p.prob, p.k, p.ks, p.Hkv, p.B, 1, &d->maps) &&
-               build_maps(p.prob, p.v, p.vs, p.Hkv, p.B, 2, &d->maps);
+               build_maps(p.prob, p.v, p.vs, p.Hkv, p.B, 2, &d->maps) &&
+               (p.prob.kind == KIND_IMG_SCATTER || p.prob.kind == KIND_IMG_GATHER0 ||
+                build_maps(p.prob, p.o, p.os, p.H, p.B, 3, &d->maps));
   *split = d->use_tma ? 0 : pick_form(p.prob, d->row_pairs, d->split_kv);
   return INTRA_OK;
 }
@@ -753,7 +758,7 @@ int intra_b200_test_tma_rows(const void* q, const void* k, const void* v, int B,
   p.q = static_cast<const __nv_bfloat16*>(q);
   p.k = static_cast<const __nv_bfloat16*>(k);
   p.v = static_cast<const __nv_bfloat16*>(v);
-  p.o = nullptr;
+  p.o = const_cast<__nv_bfloat16*>(p.q);                    // never written: the test kernel stores no output
   p.qs = {q_strides[0], q_strides[1], q_strides[2]};
   p.ks = {k_strides[0], k_strides[1], k_strides[2]};
   p.vs = {v_strides[0], v_strides[1], v_strides[2]};

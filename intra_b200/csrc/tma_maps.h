@@ -37,8 +37,9 @@ enum ViewId : int {
   VIEW_AUX = 2      // Gather-0: image-Scatter view for the keys of its text tiles
 };
 struct alignas(64) TmaMaps {
-  CUtensorMap view[3][3];   // [ViewId][query, key, value]
+  CUtensorMap view[3][4];   // [ViewId][query, key, value, output (language-model patterns, boxes of 32 rows)]
 };
+constexpr int OUT_ROWS = 32;      // rows of an output box: what one epilogue warp stages
 
 // Can the problem's tiles be fetched as TMA boxes?
 INTRA_HD bool tma_supported(const Problem& p) {
