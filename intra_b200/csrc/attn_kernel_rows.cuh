@@ -1,6 +1,6 @@
 // The attention kernel for every shape whose tiles are TMA boxes (tma_maps.h). Persistent: each CTA owns
 // one SM and walks a static list of pair tiles (intra_index.h): two 128-row query sub-tiles that share
-// every K / V tile brought into shared memory or (Gather-0) keep a K / V buffer each.
+// every K / V tile brought into shared memory or (Gather-0) share those of the text only.
 //
 // Warp roles (512 threads):
 //   warps 0-3, 4-7    softmax sets of sub-tile 0 and 1: a thread owns a query row. A set copies its scores out
@@ -164,10 +164,18 @@ __device__ __forceinline__ void issue_pv_loop(uint32_t p_tmem, uint64_t v_desc, 
   }
 }
 
+// Number of the tile buffer `x` is about to hold, counted over the CTA.
+__device__ __forceinline__ uint32_t next_fill(uint32_t (&fills)[2], uint32_t x) {
+  const uint32_t n = x ? fills[1] : fills[0];
+  fills[0] += x ? 0 : 1;
+  fills[1] += x ? 1 : 0;
+  return n;
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(const __grid_constant__ DualParams p) {
   using Cfg = RowsCfg;
-  constexpr bool SPLIT = KIND == KIND_IMG_GATHER0;         // sub-tile s has K / V buffer s to itself
+  constexpr bool SPLIT = KIND == KIND_IMG_GATHER0;         // the sub-tiles have key lists of their own
   constexpr bool IMAGE = KIND == KIND_IMG_SCATTER || KIND == KIND_IMG_GATHER0;
   enum : int {
     Q_FULL = 0, K_FULL = 2, V_FULL = 4, S_FULL = 6, PV_DONE = 10, P_FULL = 14, S_TAKEN = 16, O_DONE = 18, O_FREE = 20,
@@ -434,6 +442,9 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
       if (lane == 0) {
         for (int i = 0; i < 3; ++i) ptx::prefetch_tensormap(&p.maps.view[0][i]);
         uint32_t j = 0;                                   // key tiles requested so far by this CTA
+        // split key lists, buffers K0 K1 V0 V1: the key tile (its low two bits) whose product read it last, tiles
+        // -2 and -1 to begin with, and whether that was sub-tile 1's product
+        uint32_t used = 0xeeu, reader = 0xfu;
         ROWS_ITEMS(55)
           const int n_kv = sl.n_kv;
 #pragma unroll 1
@@ -457,15 +468,29 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
               if (!ok) break;
               fetch_kv_tile(p.maps, 2, sl.kv[0], n, sl.hk, sl.b, v_smem + st * TILE_BYTES, bar(V_FULL + st));
             } else {
-              // one K and one V buffer per sub-tile, refilled as soon as the MMA that read it has completed
+              // Image tiles: sub-tile s's own K and V go to buffer s. Text tiles are the same for both sub-tiles: one
+              // load each, to the two buffers in turn (20 loads for the 14 products of a patch item instead of 28: at four
+              // tiles per step the copies alone took 3,700 cycles, 35 B per clock and SM out of the L2). A buffer
+              // is free once the MMA that read it last has completed, sub-tile 1's where both read it.
+              const bool text = n >= sl.kv[0].text_lo && n < sl.kv[0].text_hi;
 #pragma unroll 1
               for (int i = 0; i < 4 && ok; ++i) {          // K0 (Q0) K1 (Q1) V0 V1
                 const int sx = i & 1, is_v = i >> 1;
-                ok = ROWS_WAIT((is_v ? PV_DONE : S_FULL) + 2 * sx + ((j - 1) & 1), (j - 1) >> 1, 24 + i);
-                if (!ok) break;
-                fetch_kv_tile(p.maps, 1 + is_v, sl.kv[sx], n, sl.hk, sl.b, (is_v ? v_smem : k_smem) + sx * TILE_BYTES,
-                              bar((is_v ? V_FULL : K_FULL) + sx));
-                if (n == 0 && !is_v) fetch_q_tile(p.maps, sl.q[sx], sl.h[sx], sl.b, q_smem + sx * TILE_BYTES, bar(Q_FULL + sx));
+                const uint32_t x = text ? j & 1 : uint32_t(sx);
+                if (!text || sx == 0) {
+                  const uint32_t at = x + 2 * is_v;
+                  const uint32_t last = used >> (2 * at);
+                  ok = ROWS_WAIT((is_v ? PV_DONE : S_FULL) + 2 * ((reader >> at) & 1u) + (last & 1), last >> 1, 24 + i);
+                  if (!ok) break;
+                  fetch_kv_tile(p.maps, 1 + is_v, sl.kv[sx], n, sl.hk, sl.b, (is_v ? v_smem : k_smem) + x * TILE_BYTES,
+                                bar((is_v ? V_FULL : K_FULL) + x));
+                  used = (used & ~(3u << (2 * at))) | ((j & 3u) << (2 * at));
+                  reader = (reader & ~(1u << at)) | ((text ? 1u : uint32_t(sx)) << at);
+                }
+                if (n == 0 && !is_v) {
+                  ok = ROWS_WAIT(S_FULL + 2 * sx + ((j - 1) & 1), (j - 1) >> 1, 21);
+                  if (ok) fetch_q_tile(p.maps, sl.q[sx], sl.h[sx], sl.b, q_smem + sx * TILE_BYTES, bar(Q_FULL + sx));
+                }
               }
               if (!ok) break;
             }
@@ -478,16 +503,18 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
       const uint64_t q_desc = tile_desc_kmajor(q_smem), k_desc = tile_desc_kmajor(k_smem), v_desc = tile_desc_mnmajor(v_smem);
       constexpr uint64_t kTileStep = TILE_BYTES >> 4;      // descriptor distance between buffers
       uint32_t j = 0;                                      // key tiles so far, counted over the CTA
+      uint32_t fills[2] = {0, 0};                          // split key lists: tiles buffer 0 / 1 has held before
       ROWS_ITEMS(56)
         const int n_kv = sl.n_kv;
         if (qk) {
 #pragma unroll 1
           for (int n = 0; n < n_kv && ok; ++n, ++j) {
+            const bool shared = !SPLIT || (n >= sl.kv[0].text_lo && n < sl.kv[0].text_hi);
 #pragma unroll 1
             for (int sx = 0; sx < 2; ++sx) {
-              const uint32_t st = SPLIT ? sx : j & 1;
+              const uint32_t st = shared ? j & 1 : uint32_t(sx);
               ok = (n > 0 || ROWS_WAIT(Q_FULL + sx, seq, 31)) &&
-                   ((!SPLIT && sx == 1) || ROWS_WAIT(K_FULL + st, SPLIT ? j : j >> 1, 32)) &&
+                   ((shared && sx == 1) || ROWS_WAIT(K_FULL + st, SPLIT ? next_fill(fills, st) : j >> 1, 32)) &&
                    ROWS_WAIT(S_TAKEN + (sx ^ 1), sx ? j : j - 1, 33);   // the other set has copied its scores out
               if (!ok) break;
               ptx::tc_fence_after();
@@ -501,10 +528,11 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
         } else {
 #pragma unroll 1
           for (int n = 0; n < n_kv && ok; ++n, ++j) {
+            const bool shared = !SPLIT || (n >= sl.kv[0].text_lo && n < sl.kv[0].text_hi);
 #pragma unroll 1
             for (int sx = 0; sx < 2; ++sx) {
-              const uint32_t st = SPLIT ? sx : j & 1;
-              ok = ((!SPLIT && sx == 1) || ROWS_WAIT(V_FULL + st, SPLIT ? j : j >> 1, 40)) &&
+              const uint32_t st = shared ? j & 1 : uint32_t(sx);
+              ok = ((shared && sx == 1) || ROWS_WAIT(V_FULL + st, SPLIT ? next_fill(fills, st) : j >> 1, 40)) &&
                    (n > 0 || ROWS_WAIT(O_FREE + sx, seq - 1, 37)) &&   // O of the previous item has been read
                    ROWS_WAIT(P_FULL + sx, j, 35);
               if (!ok) break;
