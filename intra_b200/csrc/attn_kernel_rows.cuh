@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
         uint32_t j = 0;                                   // key tiles requested so far by this CTA
         // split key lists, buffers K0 K1 V0 V1: the key tile (its low two bits) whose product read it last, tiles
         // -2 and -1 to begin with, and whether that was sub-tile 1's product
-        uint32_t used = 0xeeu, reader = 0xfu;
+        uint32_t used = 0xeeu, reader = 0xfu, cur = 0;
         ROWS_ITEMS(55)
           const int n_kv = sl.n_kv;
 #pragma unroll 1
@@ -468,15 +468,16 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
               if (!ok) break;
               fetch_kv_tile(p.maps, 2, sl.kv[0], n, sl.hk, sl.b, v_smem + st * TILE_BYTES, bar(V_FULL + st));
             } else {
-              // Image tiles: sub-tile s's own K and V go to buffer s. Text tiles are the same for both sub-tiles: one
-              // load each, to the two buffers in turn (20 loads for the 14 products of a patch item instead of 28: at four
+              // Image tiles: each sub-tile's own K and V. Text tiles are the same for both sub-tiles: one load each (20 loads for the 14 products of a patch item instead of 28: at four
               // tiles per step the copies alone took 3,700 cycles, 35 B per clock and SM out of the L2). A buffer
-              // is free once the MMA that read it last has completed, sub-tile 1's where both read it.
-              const bool text = n >= sl.kv[0].text_lo && n < sl.kv[0].text_hi;
+              // is free once the MMA that read it last has completed, sub-tile 1's where both read it. The next tile
+              // goes to buffer `cur`, the one that frees first: the other one after a text tile, sub-tile 0's
+              // after image tiles.
+              const bool text = is_text_tile(sl.kv[0].text, n);
 #pragma unroll 1
               for (int i = 0; i < 4 && ok; ++i) {          // K0 (Q0) K1 (Q1) V0 V1
                 const int sx = i & 1, is_v = i >> 1;
-                const uint32_t x = text ? j & 1 : uint32_t(sx);
+                const uint32_t x = cur ^ uint32_t(text ? 0 : sx);
                 if (!text || sx == 0) {
                   const uint32_t at = x + 2 * is_v;
                   const uint32_t last = used >> (2 * at);
@@ -493,6 +494,7 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
                 }
               }
               if (!ok) break;
+              cur ^= text ? 1 : 0;
             }
           }
         ROWS_ITEMS_END(1u)
@@ -503,16 +505,16 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
       const uint64_t q_desc = tile_desc_kmajor(q_smem), k_desc = tile_desc_kmajor(k_smem), v_desc = tile_desc_mnmajor(v_smem);
       constexpr uint64_t kTileStep = TILE_BYTES >> 4;      // descriptor distance between buffers
       uint32_t j = 0;                                      // key tiles so far, counted over the CTA
-      uint32_t fills[2] = {0, 0};                          // split key lists: tiles buffer 0 / 1 has held before
+      uint32_t fills[2] = {0, 0}, cur = 0;                 // split key lists: tiles buffer 0 / 1 has held before; see the requests
       ROWS_ITEMS(56)
         const int n_kv = sl.n_kv;
         if (qk) {
 #pragma unroll 1
           for (int n = 0; n < n_kv && ok; ++n, ++j) {
-            const bool shared = !SPLIT || (n >= sl.kv[0].text_lo && n < sl.kv[0].text_hi);
+            const bool shared = !SPLIT || is_text_tile(sl.kv[0].text, n);
 #pragma unroll 1
             for (int sx = 0; sx < 2; ++sx) {
-              const uint32_t st = shared ? j & 1 : uint32_t(sx);
+              const uint32_t st = SPLIT ? cur ^ uint32_t(shared ? 0 : sx) : j & 1;
               ok = (n > 0 || ROWS_WAIT(Q_FULL + sx, seq, 31)) &&
                    ((shared && sx == 1) || ROWS_WAIT(K_FULL + st, SPLIT ? next_fill(fills, st) : j >> 1, 32)) &&
                    ROWS_WAIT(S_TAKEN + (sx ^ 1), sx ? j : j - 1, 33);   // the other set has copied its scores out
@@ -524,14 +526,15 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
               }
               __syncwarp();
             }
+            cur ^= SPLIT && shared ? 1 : 0;
           }
         } else {
 #pragma unroll 1
           for (int n = 0; n < n_kv && ok; ++n, ++j) {
-            const bool shared = !SPLIT || (n >= sl.kv[0].text_lo && n < sl.kv[0].text_hi);
+            const bool shared = !SPLIT || is_text_tile(sl.kv[0].text, n);
 #pragma unroll 1
             for (int sx = 0; sx < 2; ++sx) {
-              const uint32_t st = shared ? j & 1 : uint32_t(sx);
+              const uint32_t st = SPLIT ? cur ^ uint32_t(shared ? 0 : sx) : j & 1;
               ok = ((shared && sx == 1) || ROWS_WAIT(V_FULL + st, SPLIT ? next_fill(fills, st) : j >> 1, 40)) &&
                    (n > 0 || ROWS_WAIT(O_FREE + sx, seq - 1, 37)) &&   // O of the previous item has been read
                    ROWS_WAIT(P_FULL + sx, j, 35);
@@ -544,6 +547,7 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
               }
               __syncwarp();
             }
+            cur ^= SPLIT && shared ? 1 : 0;
           }
         }
       ROWS_ITEMS_END(0xffffffffu)

@@ -282,8 +282,10 @@ INTRA_HD void q_row(const Problem& p, const Tile& t, int r, int* token, int* lo,
 // Token id held by key slot u of tile t, or -1 for a padding slot.
 //
 // Gather-0 patch-pair tiles order their slots so that each patch's keys are one contiguous
-// interval: [columns only the left patch sees | shared columns | 512 text | columns only the
-// right patch sees], image columns stored column-major (16 window rows per column).
+// interval: [8 columns | 256 text | 8 columns | 256 text | the right patch's extra columns], image columns
+// stored column-major (16 window rows per column). The left patch sees the first 768 slots, the right one starts
+// `off` columns later. Image tiles, which the two sub-tiles of an item cannot share, alternate with text tiles,
+// which they can: two image steps in a row want more bytes than the L2 delivers in their time.
 INTRA_HD int key_token(const Problem& p, const Tile& t, int u) {
   if (u < 0 || u >= t.nk) return -1;
   switch (t.kind) {
@@ -296,8 +298,10 @@ INTRA_HD int key_token(const Problem& p, const Tile& t, int u) {
       return u < TEXT_LEN ? u : img_scatter_token(p, t.g, u - TEXT_LEN);
     case KIND_IMG_GATHER0: {
       int v;
-      if (u < WIN * WIN) v = u;
-      else if (u < WIN * WIN + TEXT_LEN) return u - WIN * WIN;
+      if (u < TILE_N) v = u;
+      else if (u < TILE_N + TEXT_LEN / 2) return u - TILE_N;
+      else if (u < 2 * TILE_N + TEXT_LEN / 2) v = u - TEXT_LEN / 2;
+      else if (u < 2 * TILE_N + TEXT_LEN) return u - 2 * TILE_N;
       else v = u - TEXT_LEN;
       return TEXT_LEN + (t.r0 + v % WIN) * p.W + t.c0 + v / WIN;
     }

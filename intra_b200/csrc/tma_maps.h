@@ -61,13 +61,16 @@ struct QPlan {
   int patches;       // Gather-0: the tile is two 64-row boxes, one per 8x8 patch, the second at (c1b, c2)
   int c1b;
 };
-// The same of an item's key tiles: tiles [text_lo, text_hi) are the 512 text tokens, the others
+// The same of an item's key tiles: those in the set `text` are the text tokens in order, the others
 // (numbered without them) lie at (c1, c2) + i * (s1, s2) of view `which`.
 struct KvPlan {
   int which;
-  int text_lo, text_hi;
+  uint32_t text;
   int c1, c2, s1, s2;
 };
+constexpr uint32_t TEXT_FIRST = 0xfu;      // image-Scatter keys: the text, then the group's image tokens
+constexpr uint32_t TEXT_BETWEEN = 0x36u;   // Gather-0 patch pairs: image, 2 text, image, 2 text, image
+INTRA_HD bool is_text_tile(uint32_t text, int n) { return n < 32 && ((text >> n) & 1u); }
 
 // Grid rows of the image a tile of an image-Scatter group spans.
 INTRA_HD int img_tile_rows(const Problem& p) { return 2 * fdiv(TILE_M, p.by_quads); }
@@ -118,11 +121,10 @@ INTRA_HD QPlan plan_q(const Problem& p, const Tile& t) {
 // Key tiles of key-slot map `t`.
 INTRA_HD KvPlan plan_kv(const Problem& p, const Tile& t) {
   KvPlan k;
-  k.text_lo = k.text_hi = 0; k.s1 = 0; k.s2 = 0;
+  k.text = 0; k.s1 = 0; k.s2 = 0;
   if (t.kind == KIND_IMG_GATHER0) {
-    // slots: 16 window columns (2 tiles) | 512 text (4 tiles) | the right patch's extra columns (1 tile)
     k.which = VIEW_MAIN;
-    k.text_lo = WIN * WIN / TILE_N; k.text_hi = k.text_lo + TEXT_LEN / TILE_N;
+    k.text = TEXT_BETWEEN;
     k.c1 = t.r0; k.c2 = t.c0; k.s2 = TILE_N / WIN;
     return k;
   }
@@ -131,16 +133,22 @@ INTRA_HD KvPlan plan_kv(const Problem& p, const Tile& t) {
     case KIND_LLM_SCATTER: k.s2 = TILE_N; break;
     case KIND_LLM_GATHER1: k.s2 = fdiv(TILE_N, p.by_G); break;
     case KIND_LLM_WINDOW: k.s1 = TILE_N; break;
-    default: k.text_hi = TEXT_LEN / TILE_N; k.s2 = img_tile_rows(p); break;
+    default: k.text = TEXT_FIRST; k.s2 = img_tile_rows(p); break;
   }
   return k;
 }
 INTRA_HD void kv_box(const KvPlan& k, int n, int* which, int* c1, int* c2) {
-  const bool text = n >= k.text_lo && n < k.text_hi;
-  const int i = n < k.text_lo ? n : n - (k.text_hi - k.text_lo);
+  int t = 0;                                     // text tiles before tile n
+  const uint32_t before = n < 32 ? k.text & ((1u << n) - 1u) : k.text;
+#ifdef __CUDA_ARCH__
+  t = __popc(before);
+#else
+  for (uint32_t m = before; m != 0; m &= m - 1) ++t;
+#endif
+  const bool text = is_text_tile(k.text, n);
   *which = text ? int(VIEW_TEXT) : k.which;
-  *c1 = text ? (n - k.text_lo) * TILE_N : k.c1 + i * k.s1;
-  *c2 = text ? 0 : k.c2 + i * k.s2;
+  *c1 = text ? t * TILE_N : k.c1 + (n - t) * k.s1;
+  *c2 = text ? 0 : k.c2 + (n - t) * k.s2;
 }
 
 }  // namespace intra
