@@ -8,8 +8,9 @@
 //                     for its phase while the other set's phase runs beside it
 //   warps 8-11        epilogue: O of a finished item -> bf16 -> global while the sets are on the next item
 //   warp 12           issues QK0(j) QK1(j) over the CTA's key tiles j into the shared score buffer
-//   warp 13           one thread requests the tiles (bulk-tensor copies)
-//   warp 14           planner: decodes the CTA's items a few ahead into a ring in shared memory
+//   warp 13           one thread requests the Q and K tiles (bulk-tensor copies)
+//   warp 14           planner: decodes the CTA's items a batch ahead into shared memory; requests the V tiles (one
+//                     thread for K and V would hold up the next item's first K behind the last V's buffer)
 //   warp 15           issues PV0(j) PV1(j) as the sets deliver P (a tcgen05.mma issue blocks its thread once
 //                     ~5 MMAs are queued, so one warp for both kinds would let the queue drain in its waits)
 // TMEM: scores cols 0-127 | P0 128-191 | P1 192-255 | O0 256-383 | O1 384-511.
@@ -24,12 +25,12 @@
 //
 // Barriers: every wait is bounded (2 s) and gives up when another thread of the CTA has. Each barrier completes
 // again only after its waiter has seen the completion before, which is what lets one parity bit name a phase:
-//   s_full[s][j & 1]   QK_s of key tile j has completed. Waiters: set s; the requesting thread (K and Q buffers).
+//   s_full[s][j & 1]   QK_s of key tile j has completed. Waiters: set s; warp 13 (K and Q buffers).
 //                      QK_s(j + 2) needs s_taken of both sets for tile j + 1
 //   s_taken[s]         set s has copied its scores of a tile (4 warps). Waiter: QK warp before the other sub-tile's QK^T
 //   p_full[s]          set s has stored P of a tile (4 warps). Waiter: PV warp; the next P needs pv_done of this one
 //   pv_done[s][j & 1]  PV_s of key tile j has completed. Waiters: set s before it writes the next P or rescales O;
-//                      the requesting thread (V buffers)
+//                      warp 14 (V buffers)
 //   o_done[s], o_free[s], l_ready[s]   per item: last PV done / accumulator read / row sums published. A set
 //                      publishes an item only after o_free[s] of the item before
 //   batch_ready[r], batch_free[r]   planned items
@@ -163,6 +164,26 @@ __device__ __forceinline__ void issue_pv_loop(uint32_t p_tmem, uint64_t v_desc, 
     v_desc += 2048 >> 4;
   }
 }
+
+// Split key lists (Gather-0): which of the two K (or V) buffers the next tile goes to, and when that one is free.
+// Image tiles: each sub-tile's own. Text tiles are the same for both sub-tiles: one load for both, 20 loads for
+// the 14 products of a patch item instead of 28 (at four tiles per step the copies alone took 3,700 cycles,
+// 35 B per clock and SM out of the L2). A buffer is free once the MMA that read it last has completed, sub-tile
+// 1's where both read it. The next tile goes to buffer `cur`, the one that frees first: the other one after a text
+// tile, sub-tile 0's after image tiles.
+struct BufferUse {
+  uint32_t used = 0xeu;      // two bits per buffer: the low bits of the key tile it held last (-2 and -1 to begin with)
+  uint32_t reader = 3u;      // one bit per buffer: whether that was read last by sub-tile 1
+  uint32_t cur = 0;
+  __device__ __forceinline__ uint32_t buffer(bool shared, int sx) const { return cur ^ uint32_t(shared ? 0 : sx); }
+  __device__ __forceinline__ uint32_t barrier(uint32_t x) const { return 2 * ((reader >> x) & 1u) + ((used >> (2 * x)) & 1u); }
+  __device__ __forceinline__ uint32_t parity(uint32_t x) const { return (used >> (2 * x + 1)) & 1u; }
+  __device__ __forceinline__ void read_by(uint32_t x, uint32_t tile, int sx) {
+    used = (used & ~(3u << (2 * x))) | ((tile & 3u) << (2 * x));
+    reader = (reader & ~(1u << x)) | (uint32_t(sx) << x);
+  }
+  __device__ __forceinline__ void next(bool shared) { cur ^= shared ? 1u : 0u; }
+};
 
 // Number of the tile buffer `x` is about to hold, counted over the CTA.
 __device__ __forceinline__ uint32_t next_fill(uint32_t (&fills)[2], uint32_t x) {
@@ -420,84 +441,85 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
     if (!IMAGE && lane == 0) ptx::bulk_wait_read();        // the staging buffers live until their stores have read them
   } else {
     ptx::setmaxnreg_dec<Cfg::MMA_REGS>();
-    if (warp == 14) {
-      // ================================ planner ====================================================
-      const Problem pr = kind_problem<KIND>(p);
-      for (uint32_t batch = 0;; ++batch) {
-        const int item = dual_item_index(batch * ROW_BATCH + lane, blockIdx.x, gridDim.x);
-        const bool valid = lane < ROW_BATCH && item < p.n_items;
-        const DualItem di = dual_decode(p, pr, valid ? item : 0);
-        const uint32_t filled = __ballot_sync(0xffffffffu, valid && di.pt.kv.n_kv_tiles > 0);
-        const bool last = __popc(__ballot_sync(0xffffffffu, valid)) < ROW_BATCH;
-        RowBatch& rb = ring[batch & 1];
-        if (batch >= 2 && !ROWS_WAIT(BATCH_FREE + (batch & 1), (batch >> 1) - 1, 51)) break;
-        if ((filled >> lane) & 1u) fill_row_slot<KIND>(pr, di, rb.slot[__popc(filled & ((1u << lane) - 1u))]);
-        if (lane == 0) { rb.n = __popc(filled); rb.last = last; }
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive_at(bar(BATCH_READY + (batch & 1)));
-        if (last) break;
-      }
-    } else if (warp == 13) {
-      // ================================ requests ====================================================
+    if (warp == 13) {
+      // ================================ requests of Q and K ==========================================
       if (lane == 0) {
-        for (int i = 0; i < 3; ++i) ptx::prefetch_tensormap(&p.maps.view[0][i]);
+        for (int i = 0; i < 2; ++i) ptx::prefetch_tensormap(&p.maps.view[VIEW_MAIN][i]);
         uint32_t j = 0;                                   // key tiles requested so far by this CTA
-        // split key lists, buffers K0 K1 V0 V1: the key tile (its low two bits) whose product read it last, tiles
-        // -2 and -1 to begin with, and whether that was sub-tile 1's product
-        uint32_t used = 0xeeu, reader = 0xfu, cur = 0;
+        BufferUse use;
         ROWS_ITEMS(55)
           const int n_kv = sl.n_kv;
 #pragma unroll 1
-          for (int n = 0; n < n_kv; ++n, ++j) {
-            if (!SPLIT) {
-              // ring of two K and two V tiles; an item's queries go in between its first K and V tiles, each as
-              // early as its buffer frees
-              const uint32_t st = j & 1;
-              ok = ROWS_WAIT(S_FULL + 2 + st, (j - 2) >> 1, 22);
-              if (!ok) break;
-              fetch_kv_tile(p.maps, 1, sl.kv[0], n, sl.hk, sl.b, k_smem + st * TILE_BYTES, bar(K_FULL + st));
-              if (n == 0) {
+          for (int n = 0; n < n_kv && ok; ++n, ++j) {
+            // Each tile goes out as early as its buffer frees; an item's queries follow its first K tiles.
+            const bool shared = !SPLIT || is_text_tile(sl.kv[0].text, n);
 #pragma unroll 1
-                for (int sx = 0; sx < 2 && ok; ++sx) {
-                  ok = ROWS_WAIT(S_FULL + 2 * sx + ((j - 1) & 1), (j - 1) >> 1, 21);
-                  if (ok) fetch_q_tile(p.maps, sl.q[sx], sl.h[sx], sl.b, q_smem + sx * TILE_BYTES, bar(Q_FULL + sx));
-                }
+            for (int sx = 0; sx < 2 && ok; ++sx) {
+              if (sx == 0 || !shared) {
+                const uint32_t x = SPLIT ? use.buffer(shared, sx) : j & 1;
+                ok = SPLIT ? ROWS_WAIT(S_FULL + use.barrier(x), use.parity(x), 24 + sx) : ROWS_WAIT(S_FULL + 2 + x, (j - 2) >> 1, 22);
                 if (!ok) break;
+                fetch_kv_tile(p.maps, 1, sl.kv[SPLIT ? sx : 0], n, sl.hk, sl.b, k_smem + x * TILE_BYTES, bar(K_FULL + x));
+                if (SPLIT) use.read_by(x, j, shared ? 1 : sx);
               }
-              ok = ROWS_WAIT(PV_DONE + 2 + st, (j - 2) >> 1, 26);
-              if (!ok) break;
-              fetch_kv_tile(p.maps, 2, sl.kv[0], n, sl.hk, sl.b, v_smem + st * TILE_BYTES, bar(V_FULL + st));
-            } else {
-              // Image tiles: each sub-tile's own K and V. Text tiles are the same for both sub-tiles: one load each (20 loads for the 14 products of a patch item instead of 28: at four
-              // tiles per step the copies alone took 3,700 cycles, 35 B per clock and SM out of the L2). A buffer
-              // is free once the MMA that read it last has completed, sub-tile 1's where both read it. The next tile
-              // goes to buffer `cur`, the one that frees first: the other one after a text tile, sub-tile 0's
-              // after image tiles.
-              const bool text = is_text_tile(sl.kv[0].text, n);
-#pragma unroll 1
-              for (int i = 0; i < 4 && ok; ++i) {          // K0 (Q0) K1 (Q1) V0 V1
-                const int sx = i & 1, is_v = i >> 1;
-                const uint32_t x = cur ^ uint32_t(text ? 0 : sx);
-                if (!text || sx == 0) {
-                  const uint32_t at = x + 2 * is_v;
-                  const uint32_t last = used >> (2 * at);
-                  ok = ROWS_WAIT((is_v ? PV_DONE : S_FULL) + 2 * ((reader >> at) & 1u) + (last & 1), last >> 1, 24 + i);
-                  if (!ok) break;
-                  fetch_kv_tile(p.maps, 1 + is_v, sl.kv[sx], n, sl.hk, sl.b, (is_v ? v_smem : k_smem) + x * TILE_BYTES,
-                                bar((is_v ? V_FULL : K_FULL) + x));
-                  used = (used & ~(3u << (2 * at))) | ((j & 3u) << (2 * at));
-                  reader = (reader & ~(1u << at)) | ((text ? 1u : uint32_t(sx)) << at);
-                }
-                if (n == 0 && !is_v) {
-                  ok = ROWS_WAIT(S_FULL + 2 * sx + ((j - 1) & 1), (j - 1) >> 1, 21);
-                  if (ok) fetch_q_tile(p.maps, sl.q[sx], sl.h[sx], sl.b, q_smem + sx * TILE_BYTES, bar(Q_FULL + sx));
-                }
+              if (n == 0) {
+                ok = ROWS_WAIT(S_FULL + 2 * sx + ((j - 1) & 1), (j - 1) >> 1, 21);
+                if (ok) fetch_q_tile(p.maps, sl.q[sx], sl.h[sx], sl.b, q_smem + sx * TILE_BYTES, bar(Q_FULL + sx));
               }
-              if (!ok) break;
-              cur ^= text ? 1 : 0;
             }
+            if (SPLIT) use.next(shared);
           }
         ROWS_ITEMS_END(1u)
+      }
+    } else if (warp == 14) {
+      // ================================ planner, requests of V =======================================
+      const Problem pr = kind_problem<KIND>(p);
+      uint32_t planned = 0;                               // batches planned so far
+      bool more = true;                                   // the list goes on after them
+      auto plan = [&] {
+        const int item = dual_item_index(planned * ROW_BATCH + lane, blockIdx.x, gridDim.x);
+        const bool valid = lane < ROW_BATCH && item < p.n_items;
+        const DualItem di = dual_decode(p, pr, valid ? item : 0);
+        const uint32_t filled = __ballot_sync(0xffffffffu, valid && di.pt.kv.n_kv_tiles > 0);
+        more = __popc(__ballot_sync(0xffffffffu, valid)) == ROW_BATCH;
+        RowBatch& rb = ring[planned & 1];
+        if (planned >= 2) ok = ROWS_WAIT(BATCH_FREE + (planned & 1), (planned >> 1) - 1, 51);
+        if (!ok) return;
+        if ((filled >> lane) & 1u) fill_row_slot<KIND>(pr, di, rb.slot[__popc(filled & ((1u << lane) - 1u))]);
+        if (lane == 0) { rb.n = __popc(filled); rb.last = !more; }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_at(bar(BATCH_READY + (planned & 1)));
+        ++planned;
+      };
+      uint32_t j = 0;
+      BufferUse use;
+#pragma unroll 1
+      for (uint32_t step = 0, batch = 0, i = 0; ok; ++step) {
+        // The next batch is planned in the middle of one, when the other roles have long left the one before, or
+        // when this one is done.
+        const bool done = planned > batch && int(i) == ring[batch & 1].n;
+        if (planned == batch || (planned == batch + 1 && more && (i == 4 || done))) { plan(); continue; }
+        if (done) {
+          if (ring[batch & 1].last) break;
+          ++batch;
+          i = 0;
+          continue;
+        }
+        const RowSlot& sl = ring[batch & 1].slot[i++];
+        const int n_kv = sl.n_kv;
+#pragma unroll 1
+        for (int n = 0; n < n_kv && ok; ++n, ++j) {
+          const bool shared = !SPLIT || is_text_tile(sl.kv[0].text, n);
+#pragma unroll 1
+          for (int sx = 0; sx < (shared ? 1 : 2); ++sx) {
+            const uint32_t x = SPLIT ? use.buffer(shared, sx) : j & 1;
+            ok = SPLIT ? ROWS_WAIT(PV_DONE + use.barrier(x), use.parity(x), 26 + sx) : ROWS_WAIT(PV_DONE + 2 + x, (j - 2) >> 1, 26);
+            if (!ok) break;
+            if (lane == 0) fetch_kv_tile(p.maps, 2, sl.kv[SPLIT ? sx : 0], n, sl.hk, sl.b, v_smem + x * TILE_BYTES, bar(V_FULL + x));
+            if (SPLIT) use.read_by(x, j, shared ? 1 : sx);
+          }
+          if (SPLIT) use.next(shared);
+        }
       }
     } else {
       // ================================ MMA issue: warp 12 QK^T, warp 15 PV ==========================
