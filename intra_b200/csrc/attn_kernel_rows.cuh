@@ -31,8 +31,8 @@
 //   p_full[s]          set s has stored P of a tile (4 warps). Waiter: PV warp; the next P needs pv_done of this one
 //   pv_done[s][j & 1]  PV_s of key tile j has completed. Waiters: set s before it writes the next P or rescales O;
 //                      warp 14 (V buffers)
-//   o_done[s], o_free[s], l_ready[s]   per item: last PV done / accumulator read / row sums published. A set
-//                      publishes an item only after o_free[s] of the item before
+//   o_done[s], o_free[s], l_ready[s]   per item: last PV done / accumulator read / row sums published (two
+//                      barriers alternate)
 //   batch_ready[r], batch_free[r]   planned items
 // A wait for "the phase before the first" (parity 1 of a fresh barrier) returns at once, so the first tiles and items
 // need no special case.
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
   constexpr bool IMAGE = KIND == KIND_IMG_SCATTER || KIND == KIND_IMG_GATHER0;
   enum : int {
     Q_FULL = 0, K_FULL = 2, V_FULL = 4, S_FULL = 6, PV_DONE = 10, P_FULL = 14, S_TAKEN = 16, O_DONE = 18, O_FREE = 20,
-    L_READY = 22, BATCH_READY = 24, BATCH_FREE = 26, DRAIN = 28, N_BARS = 30
+    L_READY = 22, BATCH_READY = 26, BATCH_FREE = 28, DRAIN = 30, N_BARS = 32
   };
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bars[N_BARS];
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
     abort_flag = 0;
     for (int i = 0; i < N_BARS; ++i) {
       int n = 1;
-      if (i == P_FULL || i == P_FULL + 1 || i == S_TAKEN || i == S_TAKEN + 1 || i == L_READY || i == L_READY + 1) n = 4;
+      if (i == P_FULL || i == P_FULL + 1 || i == S_TAKEN || i == S_TAKEN + 1 || (i >= L_READY && i < L_READY + 4)) n = 4;
       if (i == O_FREE || i == O_FREE + 1) n = 4;
       if (i == BATCH_FREE || i == BATCH_FREE + 1) n = Cfg::SM_WARPS + 4 + 2 + 1;   // sets, epilogue, issuing warps, requests
       ptx::mbar_init(&bars[i], n);
@@ -361,15 +361,12 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
         if (lane == 0) ptx::mbar_arrive_at(bar(P_FULL + sx));
       }
       if (!ok) break;
-      // The epilogue warps take it from here, once they are done with this sub-tile of the item before: nothing
-      // else holds a set back over items of one key tile, and two reports would complete l_ready twice
-      // before they had looked at it.
-      ok = ROWS_WAIT(O_FREE + sx, seq - 1, 19);
-      if (!ok) break;
+      // The epilogue warps take it from here. Two barriers alternate: the report of the item after next follows the
+      // next item's PV, which waited for o_free of this one, i.e. for the epilogue to have seen this report.
       row_sum[seq & 1][sx][row] = l_run;
       if (p.f.lse != nullptr) row_max[seq & 1][sx][row] = m_run;
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive_at(bar(L_READY + sx));
+      if (lane == 0) ptx::mbar_arrive_at(bar(L_READY + 2 * sx + (seq & 1)));
     ROWS_ITEMS_END(0xffffffffu)
   } else if (warp < Cfg::SM_WARPS + 4) {
     // ================================ epilogue =====================================================
@@ -380,7 +377,7 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
 #pragma unroll 1
       for (int sx = 0; sx < 2; ++sx) {
         const int b = sl.b, h = sl.h[sx];
-        ok = ROWS_WAIT(L_READY + sx, seq, 41) && ROWS_WAIT(O_DONE + sx, seq, 43 + sx);
+        ok = ROWS_WAIT(L_READY + 2 * sx + (seq & 1), seq >> 1, 41) && ROWS_WAIT(O_DONE + sx, seq, 43 + sx);
         if (!ok) break;
         ptx::tc_fence_after();
         const float l = row_sum[seq & 1][sx][row];
