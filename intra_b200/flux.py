@@ -15,7 +15,7 @@ import math
 
 import torch
 
-from .interface import TEXT_LEN, intra_image_attn
+from .interface import TEXT_LEN, _image
 
 KERNEL_WIDTHS = (64, 128)   # latent sides of 1024^2 and 2048^2 images (intra_processor.py:30)
 
@@ -42,6 +42,4 @@ def flux_joint_attention(query, key, value, pattern: str, softmax_scale=None):
         raise ValueError("expected (batch, heads, seq, head_dim) tensors")
     width = latent_width(query.shape[2])
     scale = 1.0 / math.sqrt(query.shape[-1]) if softmax_scale is None else softmax_scale
-    out = intra_image_attn(query.transpose(1, 2), key.transpose(1, 2), value.transpose(1, 2),
-                           pattern=pattern, width=width, softmax_scale=scale)
-    return out.transpose(1, 2)
+    return _image(query, key, value, 2, 1, pattern, width, scale, True, False, None).transpose(1, 2)

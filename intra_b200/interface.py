@@ -13,7 +13,7 @@ import ctypes
 import torch
 
 from . import _loader
-from ._loader import lib, strides3
+from ._loader import lib
 
 LLM_PATTERNS = {"scatter": 0, "gather1": 1, "window": 4}
 IMAGE_PATTERNS = {"scatter": 0, "gather0": 4}
@@ -63,53 +63,120 @@ def _byte_span(x):
     return x.data_ptr(), x.data_ptr() + (last + 1) * x.element_size()
 
 
-def _empty_like(q, out=None, inputs=()):
-    """The output tensor: the caller's `out` after checks, else a fresh tensor laid out like q."""
-    if out is not None:
-        if out.shape != q.shape or out.dtype != q.dtype or out.device != q.device:
-            raise ValueError("out must match q in shape, dtype and device")
-        if out.stride(-1) != 1 or any(out.stride(d) % 8 or out.stride(d) <= 0 for d in range(3)) or out.data_ptr() % 16:
-            raise ValueError("out needs unit stride in the last dim, positive strides and 16-byte aligned rows")
-        lo, hi = _byte_span(out)
-        for x in inputs:
-            xlo, xhi = _byte_span(x)
-            if lo < xhi and xlo < hi:
-                raise ValueError("out must not overlap q, k or v: other tiles still read them while it is written")
-        return out
-    out = torch.empty_like(q)
-    if out.stride(-1) != 1 or any(out.stride(d) % 8 or out.stride(d) <= 0 for d in range(3)):
-        out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-    return out
+def _check_out(out, q, inputs):
+    """Checks of a caller's output tensor, (B, S, H, 128) like q."""
+    if out.shape != q.shape or out.dtype != q.dtype or out.device != q.device:
+        raise ValueError("out must match q in shape, dtype and device")
+    if out.stride(-1) != 1 or any(out.stride(d) % 8 or out.stride(d) <= 0 for d in range(3)) or out.data_ptr() % 16:
+        raise ValueError("out needs unit stride in the last dim, positive strides and 16-byte aligned rows")
+    lo, hi = _byte_span(out)
+    for x in inputs:
+        xlo, xhi = _byte_span(x)
+        if lo < xhi and xlo < hi:
+            raise ValueError("out must not overlap q, k or v: other tiles still read them while it is written")
 
 
-# Validated call plans, keyed by everything the checks above look at (addresses, shapes, strides,
-# dtypes, device, requires_grad). A serving loop or a layer stack calls with the same tensors over and
-# over; at S = 4096 a call is 40 us of GPU time and the checks would cost as much on the host again.
-_PLANS = {}
-_PLANS_MAX = 512
+# int64[3] constants for the C ABI by their values: building one costs as much as a tenth of a short call.
+_STRIDES = {}
+_STRIDES_MAX = 1024
 
 
-def _plan(q, k, v, out):
-    """(q, k, v, out or None, B, S, H, Hkv, q/k/v/out stride arrays or None for out) after the checks."""
-    rg = q.requires_grad or k.requires_grad or v.requires_grad
-    if rg and torch.is_grad_enabled():
+def _c_strides(batch, token, head):
+    key = (batch, token, head)
+    arr = _STRIDES.get(key)
+    if arr is None:
+        if len(_STRIDES) >= _STRIDES_MAX:
+            _STRIDES.clear()
+        arr = _STRIDES[key] = (ctypes.c_int64 * 3)(batch, token, head)
+    return arr
+
+
+def _prepare(q, k, v, token, head, out):
+    """Checks and output of a call whose q, k, v have their token and head axes at `token` and `head` (1 and 2, or
+    2 and 1). Returns (data pointers of q, k, v and the output, B, S, H, Hkv, their strides for the C ABI, the output
+    as (B, S, H, 128), and the tensors read, copies perhaps, to be held until the launch). What this function's own tests do not recognise at once goes through `_check`, which raises
+    or copies. Nothing is remembered about tensors."""
+    if (q.requires_grad or k.requires_grad or v.requires_grad) and torch.is_grad_enabled():
         raise RuntimeError("INTRA kernels are forward-only; call them under torch.no_grad()")
-    key = (q.data_ptr(), k.data_ptr(), v.data_ptr(), None if out is None else (out.data_ptr(), out.shape, out.stride(), out.dtype, out.device),
-           q.shape, k.shape, v.shape, q.stride(), k.stride(), v.stride(), q.dtype, k.dtype, v.dtype, q.device, k.device, v.device)
-    plan = _PLANS.get(key)
-    if plan is not None:
-        return (q, k, v) + plan
-    q2, k2, v2 = _check(q, k, v)
-    copied = q2 is not q or k2 is not k or v2 is not v        # fresh contiguous copies: nothing to remember
+    bf16 = torch.bfloat16
+    qn, kn = q.shape, k.shape
+    ready = False
+    if (q.is_cuda and k.is_cuda and v.is_cuda and q.dtype is bf16 and k.dtype is bf16 and v.dtype is bf16
+            and len(qn) == 4 and len(kn) == 4 and kn == v.shape and qn[3] == 128 and kn[3] == 128 and qn[0] == kn[0]
+            and qn[token] == kn[token] and kn[head] > 0 and qn[head] % kn[head] == 0
+            and k.device == q.device and v.device == q.device):
+        qs, ks, vs = q.stride(), k.stride(), v.stride()
+        ptrs = q.data_ptr(), k.data_ptr(), v.data_ptr()
+        ready = (qs[3] == 1 and ks[3] == 1 and vs[3] == 1 and not (ptrs[0] | ptrs[1] | ptrs[2]) & 15
+                 and not (qs[0] | qs[1] | qs[2] | ks[0] | ks[1] | ks[2] | vs[0] | vs[1] | vs[2]) & 7)
+    if not ready:
+        if token == 2:
+            q, k, v = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)
+            token, head = 1, 2
+        q, k, v = _check(q, k, v)
+        qn, kn = q.shape, k.shape
+        qs, ks, vs = q.stride(), k.stride(), v.stride()
+        ptrs = q.data_ptr(), k.data_ptr(), v.data_ptr()
     if out is not None:
-        _empty_like(q2, out, (q2, k2, v2))
-    B, S, H, _ = q2.shape
-    plan = (B, S, H, k2.shape[2], strides3(q2), strides3(k2), strides3(v2), None if out is None else strides3(out))
-    if not copied:
-        if len(_PLANS) >= _PLANS_MAX:
-            _PLANS.clear()
-        _PLANS[key] = plan
-    return (q2, k2, v2) + plan
+        _check_out(out, q, (q, k, v))                # only calls in (B, S, H, 128) order take `out`
+        os_ = out.stride()
+        optr = out.data_ptr()
+    else:
+        out = torch.empty_like(q)
+        os_ = out.stride()
+        if os_[3] != 1 or (os_[0] | os_[1] | os_[2]) & 7 or os_[0] <= 0 or os_[1] <= 0 or os_[2] <= 0:
+            out = torch.empty((qn[0], qn[token], qn[head], 128), dtype=bf16, device=q.device)
+            if token == 2:
+                out = out.transpose(1, 2)
+            os_ = out.stride()
+        optr = out.data_ptr()
+        if token == 2:
+            out = out.transpose(1, 2)
+    return (ptrs[0], ptrs[1], ptrs[2], optr, qn[0], qn[token], qn[head], kn[head],
+            _c_strides(qs[0], qs[token], qs[head]), _c_strides(ks[0], ks[token], ks[head]),
+            _c_strides(vs[0], vs[token], vs[head]), _c_strides(os_[0], os_[token], os_[head]), out, (q, k, v))
+
+
+def _llm(q, k, v, token, head, pattern, group_num, window, softmax_scale, strict, return_lse, out):
+    qp, kp, vp, op, B, S, H, Hkv, qs, ks, vs, os_, out, held = _prepare(q, k, v, token, head, out)
+    if strict and pattern == "gather1" and (group_num != 8 or S % (group_num * group_num)):
+        raise ValueError(f"gather1 needs group_num=8 and seqlen % 64 == 0, got G={group_num}, S={S}")
+    pid = LLM_PATTERNS[pattern]
+    dev = out.device
+    tail = (qs, ks, vs, os_, pid, int(group_num), int(window), _scale(out, softmax_scale), dev.index,
+            torch._C._cuda_getCurrentRawStream(dev.index))
+    if return_lse:
+        lse = torch.empty((B, H, S), dtype=torch.float32, device=dev)
+        rc = lib.intra_b200_fwd_llm_lse(qp, kp, vp, op, lse.data_ptr(), B, S, H, Hkv, *tail)
+    else:
+        rc = lib.intra_b200_fwd_llm(qp, kp, vp, op, B, S, H, Hkv, *tail)
+    if rc != 0:
+        _raise(rc)
+    return (out, lse) if return_lse else out
+
+
+def _image(q, k, v, token, head, pattern, width, softmax_scale, strict, return_lse, out):
+    qp, kp, vp, op, B, S, H, Hkv, qs, ks, vs, os_, out, held = _prepare(q, k, v, token, head, out)
+    if not strict and (width < 16 or width % 8):
+        raise ValueError("width must be a multiple of 8 and at least 16")
+    if strict and width not in (64, 128):
+        raise ValueError("image kernels are compiled for width 64 and 128")
+    if S != TEXT_LEN + width * width:
+        raise ValueError(f"expected {TEXT_LEN} text + {width}x{width} image tokens, got {S}")
+    if Hkv != H:
+        raise ValueError("image attention is multi-head: k/v need as many heads as q")
+    pid = IMAGE_PATTERNS[pattern]
+    dev = out.device
+    tail = (qs, ks, vs, os_, pid, int(width), _scale(out, softmax_scale), dev.index,
+            torch._C._cuda_getCurrentRawStream(dev.index))
+    if return_lse:
+        lse = torch.empty((B, H, S), dtype=torch.float32, device=dev)
+        rc = lib.intra_b200_fwd_image_lse(qp, kp, vp, op, lse.data_ptr(), B, S, H, *tail)
+    else:
+        rc = lib.intra_b200_fwd_image(qp, kp, vp, op, B, S, H, *tail)
+    if rc != 0:
+        _raise(rc)
+    return (out, lse) if return_lse else out
 
 
 def intra_llm_attn(q, k, v, pattern="scatter", group_num=8, window=576, softmax_scale=None, *, strict=True,
@@ -128,25 +195,7 @@ def intra_llm_attn(q, k, v, pattern="scatter", group_num=8, window=576, softmax_
     denominator, which is what merging attention over disjoint key sets needs. `out=` (not in the
     reference, which always allocates) writes into a tensor of the caller's; it must not alias q, k, v.
     """
-    q, k, v, B, S, H, Hkv, qs, ks, vs, os_ = _plan(q, k, v, out)
-    if strict and pattern == "gather1" and (group_num != 8 or S % (group_num * group_num)):
-        raise ValueError(f"gather1 needs group_num=8 and seqlen % 64 == 0, got G={group_num}, S={S}")
-    pid = LLM_PATTERNS[pattern]
-    if out is None:
-        out = _empty_like(q)
-        os_ = strides3(out)
-    dev = q.device
-    tail = (qs, ks, vs, os_, pid, int(group_num), int(window), _scale(q, softmax_scale), dev.index,
-            torch.cuda.current_stream(dev).cuda_stream)
-    if return_lse:
-        lse = torch.empty((B, H, S), dtype=torch.float32, device=dev)
-        rc = lib.intra_b200_fwd_llm_lse(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
-                                        B, S, H, Hkv, *tail)
-    else:
-        rc = lib.intra_b200_fwd_llm(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, S, H, Hkv, *tail)
-    if rc != 0:
-        _raise(rc)
-    return (out, lse) if return_lse else out
+    return _llm(q, k, v, 1, 2, pattern, group_num, window, softmax_scale, strict, return_lse, out)
 
 
 def intra_image_attn(q, k, v, pattern="scatter", width=64, softmax_scale=None, *, strict=True, return_lse=False,
@@ -162,31 +211,7 @@ def intra_image_attn(q, k, v, pattern="scatter", width=64, softmax_scale=None, *
     the reference) accepts any width that is a multiple of 8 and at least 16. `return_lse=True` returns
     `(out, lse)` and `out=` writes into the caller's tensor, as in intra_llm_attn.
     """
-    q, k, v, B, S, H, Hkv, qs, ks, vs, os_ = _plan(q, k, v, out)
-    if not strict and (width < 16 or width % 8):
-        raise ValueError("width must be a multiple of 8 and at least 16")
-    if strict and width not in (64, 128):
-        raise ValueError("image kernels are compiled for width 64 and 128")
-    if S != TEXT_LEN + width * width:
-        raise ValueError(f"expected {TEXT_LEN} text + {width}x{width} image tokens, got {S}")
-    if Hkv != H:
-        raise ValueError("image attention is multi-head: k/v need as many heads as q")
-    pid = IMAGE_PATTERNS[pattern]
-    if out is None:
-        out = _empty_like(q)
-        os_ = strides3(out)
-    dev = q.device
-    tail = (qs, ks, vs, os_, pid, int(width), _scale(q, softmax_scale), dev.index,
-            torch.cuda.current_stream(dev).cuda_stream)
-    if return_lse:
-        lse = torch.empty((B, H, S), dtype=torch.float32, device=dev)
-        rc = lib.intra_b200_fwd_image_lse(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
-                                          B, S, H, *tail)
-    else:
-        rc = lib.intra_b200_fwd_image(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, S, H, *tail)
-    if rc != 0:
-        _raise(rc)
-    return (out, lse) if return_lse else out
+    return _image(q, k, v, 1, 2, pattern, width, softmax_scale, strict, return_lse, out)
 
 
 def decode_attn(q, k, v, mask=None, softmax_scale=None):

@@ -17,7 +17,7 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
-from .interface import decode_attn, intra_llm_attn
+from .interface import _llm, decode_attn
 
 NUM_GROUPS = 8          # intra_token_attn.py:22-24
 WINDOW_BACK = 512
@@ -51,12 +51,9 @@ def make_intra_attention(num_groups: int = NUM_GROUPS, back: int = WINDOW_BACK, 
             o = F.scaled_dot_product_attention(query, k2, v2, attn_mask=am, scale=scaling, is_causal=False)
             return o.transpose(1, 2).contiguous(), None
         mt = force_masktype if force_masktype is not None else layer_masktype(getattr(module, "layer_idx", 0))
-        q, k, v = (x.transpose(1, 2) for x in (query, key, value))
-        with torch.no_grad():
-            if mt == 0:
-                out = intra_llm_attn(q, k, v, "scatter", group_num=num_groups, softmax_scale=scaling)
-            else:
-                out = intra_llm_attn(q, k, v, "window", window=window, softmax_scale=scaling)
+        if torch.is_grad_enabled():          # the kernels are forward-only; this callable is, too
+            query, key, value = query.detach(), key.detach(), value.detach()
+        out = _llm(query, key, value, 2, 1, "scatter" if mt == 0 else "window", num_groups, window, scaling, True, False, None)
         return out, None
 
     return intra_attention_forward
