@@ -526,7 +526,7 @@ def run_ours(args):
                     "ms_per_step": e2e_ms / e_steps if e_steps else None},
             "gpu_launches": args.steps * len(calls),
             "clocks": clocks.summary(),
-            "roofline": {"bound": "tensor", "kernel": "intra_fwd_dual_kernel (%s/%s launch)" % (calls[dom][0], calls[dom][1]),
+            "roofline": {"bound": "tensor", "kernel": "intra_fwd_rows_kernel (%s/%s launch)" % (calls[dom][0], calls[dom][1]),
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_source": peaks_kind + " bf16_tflops (burst)",
                          "frac_of_sustained": achieved / sustained,
