@@ -11,7 +11,10 @@ struct DualParams {
   int n_pair_tiles;     // pair tiles per (batch, head or head pair)
   int heads_per_item;   // row_pairs ? H : H / 2  (number of items per pair tile and batch)
   int n_items;          // n_pair_tiles * B * heads_per_item
-  FastDiv by_tile, by_heads, by_rep;   // B * heads_per_item, heads_per_item, H / Hkv
+  int last_wave;        // waves alternate between heaviest and lightest first; the last one ends with the lightest
+  // Items are numbered wave by wave (plan_launch), within a wave pair tile by pair tile: divisors items per wave,
+  // (batch, head) combinations per wave, heads_per_item, H / Hkv.
+  FastDiv by_wave, by_tile, by_heads, by_rep;
   int split_kv;         // the two sub-tiles keep their own key lists (Gather-0): K / V buffer s belongs to sub-tile s
   int use_tma;          // tiles are fetched as TMA boxes (tma_maps.h) instead of cp.async row gathers
   int wide_stores;      // every output row is 32-byte aligned: 256-bit global stores
@@ -30,8 +33,11 @@ INTRA_HD int dual_item_index(int seq, int cta, int n_cta) {
 
 INTRA_HD DualItem dual_decode(const DualParams& p, const Problem& prob, int item) {
   DualItem it;
-  const int idx = fdiv(item, p.by_tile);
-  const int rem = item - idx * int(p.by_tile.d);
+  const int wave = fdiv(item, p.by_wave);
+  const int in_wave = item - wave * int(p.by_wave.d);
+  int idx = fdiv(in_wave, p.by_tile);
+  const int rem = wave * int(p.by_tile.d) + in_wave - idx * int(p.by_tile.d);
+  if ((p.last_wave - wave) & 1) idx = p.n_pair_tiles - 1 - idx;
   it.b = fdiv(rem, p.by_heads);
   const int hh = rem - it.b * p.heads_per_item;
   if (p.row_pairs) { it.h0 = it.h1 = hh; } else { it.h0 = 2 * hh; it.h1 = 2 * hh + 1; }

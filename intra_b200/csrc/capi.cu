@@ -316,7 +316,21 @@ int plan_launch(const FwdParams& p, DualParams* d, int* split) {
   const int64_t items = int64_t(d->n_pair_tiles) * p.B * d->heads_per_item;
   if (items <= 0 || items > 0x7fffffffLL) return INTRA_ERR_UNSUPPORTED;
   d->n_items = static_cast<int>(items);
-  d->by_tile = fast_div(p.B * d->heads_per_item);
+  // All (batch, head) combinations run through the pair tiles, heaviest first, together - unless a grouped pattern's
+  // K and V are larger than the L2: every level of row tiles then reads all of them from HBM again (7.0 GB per
+  // launch at 65536 tokens and 8 KV heads, 1.3 GB compulsory). One KV head at a time, its K and V stay. GPU time of
+  // Scatter G=8, 32/8 heads, 65536 tokens 3431 -> 3178 us (back to back under the power cap 3800 -> 3505), of which
+  // waves that all run from heavy to light, 6 % out of balance, gave half (3467 -> 3325; 46000 tokens 1729 -> 1632,
+  // 32768 (134 MB) 892 -> 874, 32/32 heads 32768 1058 -> 966). Smaller ones only lose balance: G=2 23000 tokens
+  // (94 MB) 1585 -> 1687.
+  constexpr int64_t L2_BYTES = 126ll << 20;
+  const bool grouped = p.prob.kind == KIND_LLM_SCATTER || p.prob.kind == KIND_LLM_GATHER1;
+  const int64_t kv_bytes = int64_t(p.B) * p.prob.S * p.Hkv * (2 * HEAD_DIM * 2);
+  const int per_kv_head = d->row_pairs ? p.H / p.Hkv : p.H / p.Hkv / 2;
+  const int combos = grouped && kv_bytes > L2_BYTES ? per_kv_head : p.B * d->heads_per_item;
+  d->by_wave = fast_div(d->n_pair_tiles * combos);
+  d->by_tile = fast_div(combos);
+  d->last_wave = p.B * d->heads_per_item / combos - 1;
   d->by_heads = fast_div(d->heads_per_item);
   d->by_rep = fast_div(p.H / p.Hkv);
   d->wide_stores = (reinterpret_cast<uintptr_t>(p.o) % 32 == 0 && p.os.sb % 16 == 0 && p.os.ss % 16 == 0 && p.os.sh % 16 == 0) ? 1 : 0;
