@@ -81,7 +81,8 @@ struct Problem {
 // Length of group g's packed token list for the two grouped LLM patterns.
 INTRA_HD int llm_group_len(const Problem& p, int kind, int g) {
   if (kind == KIND_LLM_SCATTER) return p.n_base + (g < p.n_longer ? 1 : 0);
-  return p.n_base + imin(imax(p.n_rem - g * p.G, 0), p.G);
+  const int64_t left = int64_t(p.n_rem) - int64_t(g) * p.G;      // of the last, partial span from this group's segment on
+  return p.n_base + int(left < 0 ? 0 : left < p.G ? left : p.G);
 }
 
 // Token id of packed index t in group g.
@@ -121,6 +122,7 @@ INTRA_HD int make_problem(int kind, int S, int G, int W, Problem* out) {
         p.n_rem = int(S % span);
       }
       p.tiles_m = ceil_div(llm_group_len(p, kind, 0), TILE_M);     // no group is longer than the first
+      if (int64_t(p.tiles_m) * G > 0x7fffffff) return -1;
       p.n_tiles = p.tiles_m * G;
       break;
     }

@@ -98,3 +98,20 @@ def test_odd_image_widths_visit_exactly_the_mask(lib, width):
     S = 512 + width * width
     _check_random_shape(lib, "image", "scatter", S, width)
     _check_random_shape(lib, "image", "gather0", S, width)
+
+
+@pytest.mark.parametrize("S,G", [(60001, 50000), (46341, 46341), (92681, 46340)])
+def test_gather1_group_products_beyond_32_bits(lib, S, G):
+    """Gather-1 with so many groups that group * segment length passes 2^31: every token is still in one tile, with
+    the tokens of its segment up to it as keys."""
+    nt, nkv = ctypes.c_int64(0), ctypes.c_int64(0)
+    assert lib.intra_b200_tile_counts(0, 1, S, G, ctypes.byref(nt), ctypes.byref(nkv)) == 0
+    tiles = [-(-min(G, S - first) // 128) for first in range(0, S, G)]
+    assert nt.value == sum(tiles)
+    assert nkv.value == sum(n * (n + 1) // 2 for n in tiles)
+
+
+def test_gather1_with_more_tiles_than_can_be_numbered_is_refused(lib):
+    """One long group among so many that groups * tiles of the longest passes 2^31."""
+    nt, nkv = ctypes.c_int64(0), ctypes.c_int64(0)
+    assert lib.intra_b200_tile_counts(0, 1, 800000, 800000, ctypes.byref(nt), ctypes.byref(nkv)) == -2
