@@ -132,7 +132,7 @@ INTRA_HD int make_problem(int kind, int S, int G, int W, Problem* out) {
       break;
     case KIND_IMG_SCATTER:
     case KIND_IMG_GATHER0:
-      if (W < 16 || W % 8 != 0 || S != TEXT_LEN + W * W) return -1;
+      if (W < 16 || W % 8 != 0 || S != TEXT_LEN + int64_t(W) * W) return -1;
       p.G = IMG_GROUPS;
       p.n_img = W * W / IMG_GROUPS;
       p.tiles_m = 1 + ceil_div(p.n_img, TILE_M);

@@ -115,3 +115,10 @@ def test_gather1_with_more_tiles_than_can_be_numbered_is_refused(lib):
     """One long group among so many that groups * tiles of the longest passes 2^31."""
     nt, nkv = ctypes.c_int64(0), ctypes.c_int64(0)
     assert lib.intra_b200_tile_counts(0, 1, 800000, 800000, ctypes.byref(nt), ctypes.byref(nkv)) == -2
+
+
+def test_image_widths_whose_square_wraps_are_refused(lib):
+    """65536 * 65536 is 0 in 32 bits: such a grid must not pass for an image of no tokens."""
+    nt, nkv = ctypes.c_int64(0), ctypes.c_int64(0)
+    for pattern in (0, 4):
+        assert lib.intra_b200_tile_counts(1, pattern, 512, 65536, ctypes.byref(nt), ctypes.byref(nkv)) == -2
