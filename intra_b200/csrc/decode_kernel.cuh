@@ -88,6 +88,9 @@ __device__ __forceinline__ void split_bf16(float p0, float p1, uint32_t& hi, uin
   hi = ptx::pack_bf16(p0, p1);
   lo = ptx::pack_bf16(p0 - __uint_as_float(hi << 16), p1 - __uint_as_float(hi & 0xffff0000u));
 }
+// Sum of the results of P's high and low parts. An infinite value row makes the high one infinite (or NaN, where
+// infinities meet); the low one, a rounding error of either sign or zero times infinity, must not turn it into NaN.
+__device__ __forceinline__ float join_parts(float hi, float lo) { return fabsf(hi) < CUDART_INF_F ? hi + lo : hi; }
 // Factor that brings a partial result taken against maximum m to maximum m_all (0 for an empty one).
 __device__ __forceinline__ float merge_weight(float m, float m_all) {
   return m == -CUDART_INF_F ? 0.f : ptx::ex2(m - m_all);
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS_PER_SM) decode_kernel(co
 #pragma unroll
   for (int t = 0; t < 16; ++t)
     *reinterpret_cast<float2*>(part_o + (warp * DEC_HEADS + g) * ROW + 8 * t + 2 * j) =
-        make_float2(o[t][0] + o[t][2], o[t][1] + o[t][3]);
+        make_float2(join_parts(o[t][0], o[t][2]), join_parts(o[t][1], o[t][3]));
   __syncthreads();
   for (int h = 0; h < n_heads; ++h) {                              // thread = dim
     float m_all = -CUDART_INF_F;

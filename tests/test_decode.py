@@ -104,6 +104,17 @@ def test_decode_kernel_masked_keys_and_special_values():
     k3[0, :, 50] = float("nan")                                # a visible NaN reaches every head of its batch entry only
     out = decode_attn(q, k3, v)
     assert bool(out[0].isnan().all()) and bool(torch.isfinite(out[1]).all())
+    v3 = v.clone()                                             # visible infinities stay infinities, in their dimension only
+    v3[0, 0, 50, 5], v3[0, 1, 7, 9], v3[1, 0, 0, 127] = float("inf"), float("-inf"), float("-inf")
+    out = decode_attn(q, k, v3)
+    ref, spread = _reference(q, k, v3, None, 128 ** -0.5)
+    finite = ref.isfinite()
+    assert int((~finite).sum()) == 3 * 4 and torch.equal(out.double()[~finite], ref[~finite])
+    assert float(((out.double() - ref).abs() - (2.0 ** -8 * ref.abs() + 2.0 ** -14 * spread))[finite].max()) <= 0
+    v3[0, 0, 60, 5] = float("-inf")                            # both signs: undefined
+    assert bool(decode_attn(q, k, v3)[0, 0, :4, 5].isnan().all())
+    one = decode_attn(q[:1], k[:1, :, :1], v3[1:, :, :1])      # a single key: its probability is exactly one
+    assert torch.equal(one[0, 0], v3[1, :, 0].repeat_interleave(4, 0))
     big = decode_attn(q * 50, k, v)                            # near one-hot rows
     ref, spread = _reference(q * 50, k, v, None, 128 ** -0.5)
     assert float(((big.double() - ref).abs() - (2.0 ** -8 * ref.abs() + 2.0 ** -11 * spread)).max()) <= 0   # fp32 scores of several hundred
