@@ -43,8 +43,11 @@ std::atomic<int> g_force_no_tma{0};      // 1: cp.async row gathers even where T
 constexpr int ROW_OWNER_MIN_TILES = 8;
 std::atomic<int> g_force_split{0};       // 1 (row-owner form), 2 or 4: its softmax column split; 0: the launcher decides
 
+// Every failure is reported once: the runtime's own record of it is cleared, or the check after the next launch
+// would report it again.
 int cuda_fail(cudaError_t e) {
   g_last_cuda_error = static_cast<int>(e);
+  cudaGetLastError();
   return INTRA_ERR_CUDA;
 }
 

@@ -1,9 +1,12 @@
 """One-token decode of the transformers-style backend: the decode kernel against fp64 attention and against
 the SDPA call it stands in for, over the forms of cache and mask it takes; what it leaves to SDPA."""
+import ctypes
+
 import pytest
 import torch
 import torch.nn.functional as F
 
+from intra_b200 import intra_llm_attn
 from intra_b200.interface import decode_attn
 from intra_b200.llm_backend import make_intra_attention
 
@@ -138,6 +141,36 @@ def test_decode_kernel_under_capture_and_on_other_streams():
     graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.gpu
+def test_a_failed_launch_is_reported_once(lib):
+    """A decode launch that the runtime refuses (on a stream whose capture has been invalidated) returns its error; the
+    next attention call on the thread succeeds."""
+    q, k, v = _inputs(1, 32, 8, 100)
+    want, out = decode_attn(q, k, v), torch.empty(1, 1, 32, 128, dtype=torch.bfloat16, device="cuda")
+    prompt = torch.randn(1, 64, 4, 128, device="cuda").bfloat16()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    rt = ctypes.CDLL("libcudart.so.%s" % torch.version.cuda.split(".")[0])        # the runtime torch has loaded
+    raw, graph, need = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p(), ctypes.c_int64(0)
+
+    def decode(s):
+        return lib.intra_b200_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), None, out.data_ptr(), None, 0, need, 1, 100, 32, 8,
+                                     *q.stride()[:2], k.stride(0), k.stride(2), k.stride(1), v.stride(0), v.stride(2), v.stride(1),
+                                     0, 0, 128 ** -0.5, 0, s)
+
+    assert rt.cudaStreamBeginCapture(raw, 2) == 0                                   # 2: this thread may call anything meanwhile
+    assert rt.cudaStreamSynchronize(raw) != 0                                       # not allowed: the capture is invalid now
+    rc = decode(raw)
+    assert rt.cudaStreamEndCapture(raw, ctypes.byref(graph)) != 0
+    rt.cudaGetLastError()
+    assert rc == -4 and lib.intra_b200_last_cuda_error() != 0
+    with torch.no_grad():
+        assert bool(torch.isfinite(intra_llm_attn(prompt, prompt, prompt, "window")).all())
+    assert decode(None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
 
 
 @pytest.mark.gpu
