@@ -217,7 +217,7 @@ def intra_image_attn(q, k, v, pattern="scatter", width=64, softmax_scale=None, *
 def decode_attn(q, k, v, mask=None, softmax_scale=None):
     """Dense attention of one token per sequence over its cache: q (B, H, 1, 128), k and v
     (B, Hkv, S, 128), `mask` None or bool (B or 1, 1, 1, >= S), nonzero = visible. Returns (B, 1, H, 128), or None
-    for calls the decode kernel does not take - other types, devices, layouts or broadcasts, masks per
+    for calls the decode kernel does not take - other types, GPUs, layouts or broadcasts, masks per
     head or additive, and everything that looks inside an operator (autograd, forward-mode, vmap, tracing,
     dispatch modes, autocast to another type) - which are the caller's to run as torch operators."""
     if type(q) is not torch.Tensor or type(k) is not torch.Tensor or type(v) is not torch.Tensor:
@@ -261,6 +261,8 @@ def decode_attn(q, k, v, mask=None, softmax_scale=None):
             break
         nbytes = need.value
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    if rc == _loader.ERR_DEVICE:                     # another GPU than the kernels are built for
+        return None
     if rc != 0:
         _raise(rc)
     return out

@@ -6,7 +6,7 @@ import pytest
 import torch
 import torch.nn.functional as F
 
-from intra_b200 import intra_llm_attn
+from intra_b200 import interface, intra_llm_attn
 from intra_b200.interface import decode_attn
 from intra_b200.llm_backend import make_intra_attention
 
@@ -196,6 +196,19 @@ def test_calls_the_decode_kernel_leaves_to_sdpa():
         assert decode_attn(q, k, v) is None and fn(None, q, k, v)[0].dtype == torch.float16
     batched = torch.vmap(lambda a, b, c: fn(None, a, b, c)[0])(q[None], k[None], v[None])
     assert float((batched[0].float() - decode_attn(q, k, v).float()).abs().max()) <= 1.6e-2
+
+
+@pytest.mark.gpu
+def test_decode_on_another_gpu_is_sdpa(monkeypatch):
+    """The library refuses devices that are not sm_100; the step runs there as torch operators."""
+    class Refuses:
+        intra_b200_decode = staticmethod(lambda *args: -5)
+
+    q, k, v = _inputs(2, 8, 2, 64)
+    monkeypatch.setattr(interface, "lib", Refuses)
+    want = F.scaled_dot_product_attention(q, k.repeat_interleave(4, 1), v.repeat_interleave(4, 1)).transpose(1, 2)
+    assert decode_attn(q, k, v) is None
+    assert torch.equal(make_intra_attention()(None, q, k, v)[0], want)
 
 
 def test_decode_on_the_cpu_is_sdpa():
