@@ -20,6 +20,31 @@ IMAGE_PATTERNS = {"scatter": 0, "gather0": 4}
 TEXT_LEN = 512
 
 
+def _torch_name(path):
+    """torch.<path>, or None where this release of torch has no such name."""
+    obj = torch
+    for part in path.split("."):
+        obj = getattr(obj, part, None)
+    return obj
+
+
+# What torch keeps under private names: the current stream's handle, and whatever looks inside operators.
+_raw_stream = _torch_name("_C._cuda_getCurrentRawStream") or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+_tracing_state = _torch_name("_C._get_tracing_state")
+_dispatch_modes = _torch_name("_C._len_torch_dispatch_stack")
+_functorch_level = _torch_name("_C._functorch.peek_interpreter_stack")
+_forward_ad = _torch_name("autograd.forward_ad")
+
+
+def _watched():
+    """Does something look inside the operators that are called now: tracing, a dispatch mode, vmap and its like,
+    forward-mode? True, too, where this release of torch does not tell."""
+    if _tracing_state is None or _dispatch_modes is None or _functorch_level is None:
+        return True
+    return (_tracing_state() is not None or _dispatch_modes() > 0 or _functorch_level() is not None
+            or getattr(_forward_ad, "_current_level", 0) >= 0)
+
+
 def _check(q, k, v):
     """Argument checks of the reference (intra_attn/interface.py:17-23), plus the layout the
     library needs: the reference's kernels silently assume 128-element head stride and equal q/k row
@@ -144,7 +169,7 @@ def _llm(q, k, v, token, head, pattern, group_num, window, softmax_scale, strict
     pid = LLM_PATTERNS[pattern]
     dev = out.device
     tail = (qs, ks, vs, os_, pid, int(group_num), int(window), _scale(out, softmax_scale), dev.index,
-            torch._C._cuda_getCurrentRawStream(dev.index))
+            _raw_stream(dev.index))
     if return_lse:
         lse = torch.empty((B, H, S), dtype=torch.float32, device=dev)
         rc = lib.intra_b200_fwd_llm_lse(qp, kp, vp, op, lse.data_ptr(), B, S, H, Hkv, *tail)
@@ -168,7 +193,7 @@ def _image(q, k, v, token, head, pattern, width, softmax_scale, strict, return_l
     pid = IMAGE_PATTERNS[pattern]
     dev = out.device
     tail = (qs, ks, vs, os_, pid, int(width), _scale(out, softmax_scale), dev.index,
-            torch._C._cuda_getCurrentRawStream(dev.index))
+            _raw_stream(dev.index))
     if return_lse:
         lse = torch.empty((B, H, S), dtype=torch.float32, device=dev)
         rc = lib.intra_b200_fwd_image_lse(qp, kp, vp, op, lse.data_ptr(), B, S, H, *tail)
@@ -226,9 +251,7 @@ def decode_attn(q, k, v, mask=None, softmax_scale=None):
         return None
     if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
         return None
-    if (torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None
-            or torch._C._len_torch_dispatch_stack() or torch._C._functorch.peek_interpreter_stack() is not None
-            or torch.autograd.forward_ad._current_level >= 0 or q.is_neg() or k.is_neg() or v.is_neg()
+    if (torch.compiler.is_compiling() or _watched() or q.is_neg() or k.is_neg() or v.is_neg()
             or (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.bfloat16)):
         return None
     dev = q.device
@@ -256,7 +279,7 @@ def decode_attn(q, k, v, mask=None, softmax_scale=None):
         rc = lib.intra_b200_decode(qp, kp, vp, mp, out.data_ptr(), None if scratch is None else scratch.data_ptr(), nbytes,
                                    need, B, S, H, Hkv, qs[0], qs[1], ks[0], ks[2], ks[1], vs[0], vs[2], vs[1], ms0, ms1,
                                    0.08838834764831845 if softmax_scale is None else softmax_scale, dev.index,
-                                   torch._C._cuda_getCurrentRawStream(dev.index))
+                                   _raw_stream(dev.index))
         if rc != _loader.NEED_SCRATCH:
             break
         nbytes = need.value

@@ -211,6 +211,32 @@ def test_decode_on_another_gpu_is_sdpa(monkeypatch):
     assert torch.equal(make_intra_attention()(None, q, k, v)[0], want)
 
 
+@pytest.mark.parametrize("name", ["_tracing_state", "_dispatch_modes", "_functorch_level", "_forward_ad"])
+def test_a_torch_without_a_private_name_is_taken_to_be_watching(monkeypatch, name):
+    assert not interface._watched()
+    monkeypatch.setattr(interface, name, None)
+    assert interface._watched()
+
+
+def test_names_torch_does_not_have():
+    assert interface._torch_name("_C._no_such_name") is None and interface._torch_name("no_module.no_name") is None
+    assert interface._torch_name("nn.functional.scaled_dot_product_attention") is F.scaled_dot_product_attention
+
+
+@pytest.mark.gpu
+def test_decode_without_torchs_private_names(monkeypatch):
+    q, k, v = _inputs(2, 8, 2, 64)
+    want = decode_attn(q, k, v)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        assert interface._raw_stream(0) == side.cuda_stream
+    monkeypatch.setattr(interface, "_raw_stream", lambda index: torch.cuda.current_stream(index).cuda_stream)
+    assert torch.equal(decode_attn(q, k, v), want)
+    monkeypatch.setattr(interface, "_functorch_level", None)
+    sdpa = F.scaled_dot_product_attention(q, k.repeat_interleave(4, 1), v.repeat_interleave(4, 1)).transpose(1, 2)
+    assert torch.equal(make_intra_attention()(None, q, k, v)[0], sdpa)
+
+
 def test_decode_on_the_cpu_is_sdpa():
     q, k, v = _inputs(2, 8, 2, 30, device="cpu")
     m = _mask("random", 2, 30, device="cpu")
