@@ -34,12 +34,21 @@ _tracing_state = _torch_name("_C._get_tracing_state")
 _dispatch_modes = _torch_name("_C._len_torch_dispatch_stack")
 _functorch_level = _torch_name("_C._functorch.peek_interpreter_stack")
 _forward_ad = _torch_name("autograd.forward_ad")
+_function_modes = _torch_name("_C._len_torch_function_stack")
+_function_mode_stack = _torch_name("overrides._get_current_function_mode_stack")
+try:
+    from torch.utils._device import DeviceContext as _device_context
+except ImportError:
+    _device_context = None
 
 
 def _watched():
-    """Does something look inside the operators that are called now: tracing, a dispatch mode, vmap and its like,
-    forward-mode? True, too, where this release of torch does not tell."""
-    if _tracing_state is None or _dispatch_modes is None or _functorch_level is None:
+    """Does something look at the operators that are called now: tracing, a dispatch or function mode, vmap and its like,
+    forward-mode? True, too, where this release of torch does not tell. A default device is a function mode that only
+    places new tensors."""
+    if _tracing_state is None or _dispatch_modes is None or _functorch_level is None or _function_modes is None:
+        return True
+    if _function_modes() > 0 and (_function_mode_stack is None or any(type(m) is not _device_context for m in _function_mode_stack())):
         return True
     return (_tracing_state() is not None or _dispatch_modes() > 0 or _functorch_level() is not None
             or getattr(_forward_ad, "_current_level", 0) >= 0)

@@ -5,6 +5,7 @@ import ctypes
 import pytest
 import torch
 import torch.nn.functional as F
+from torch.overrides import TorchFunctionMode
 
 from intra_b200 import interface, intra_llm_attn
 from intra_b200.interface import decode_attn
@@ -211,11 +212,43 @@ def test_decode_on_another_gpu_is_sdpa(monkeypatch):
     assert torch.equal(make_intra_attention()(None, q, k, v)[0], want)
 
 
-@pytest.mark.parametrize("name", ["_tracing_state", "_dispatch_modes", "_functorch_level", "_forward_ad"])
+@pytest.mark.parametrize("name", ["_tracing_state", "_dispatch_modes", "_functorch_level", "_forward_ad", "_function_modes"])
 def test_a_torch_without_a_private_name_is_taken_to_be_watching(monkeypatch, name):
     assert not interface._watched()
     monkeypatch.setattr(interface, name, None)
     assert interface._watched()
+
+
+class _Calls(TorchFunctionMode):
+    """Notes the functions that are called under it."""
+
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        self.seen.append(func)
+        return func(*args, **(kwargs or {}))
+
+
+def test_function_modes_watch_and_default_devices_do_not():
+    with torch.device("cpu"):
+        assert not interface._watched()
+        with _Calls():
+            assert interface._watched()
+    with _Calls(), torch.device("cpu"):
+        assert interface._watched()
+
+
+@pytest.mark.gpu
+def test_a_function_mode_sees_the_decode_step():
+    q, k, v = _inputs(2, 8, 2, 64)
+    want = decode_attn(q, k, v)
+    with torch.device("cuda"):
+        assert torch.equal(decode_attn(q, k, v), want)
+    with _Calls() as calls:
+        make_intra_attention()(None, q, k, v)
+    assert F.scaled_dot_product_attention in calls.seen
 
 
 def test_names_torch_does_not_have():
