@@ -9,6 +9,7 @@ they divide the query heads. Forward only.
 from __future__ import annotations
 
 import ctypes
+import numbers
 
 import torch
 
@@ -259,6 +260,8 @@ def decode_attn(q, k, v, mask=None, softmax_scale=None):
     if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16 or not q.is_cuda:
         return None
     if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
+        return None
+    if softmax_scale is not None and type(softmax_scale) is not float and not isinstance(softmax_scale, numbers.Real):
         return None
     if (torch.compiler.is_compiling() or _watched() or q.is_neg() or k.is_neg() or v.is_neg()
             or (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.bfloat16)):

@@ -2,6 +2,7 @@
 the SDPA call it stands in for, over the forms of cache and mask it takes; what it leaves to SDPA."""
 import ctypes
 
+import numpy as np
 import pytest
 import torch
 import torch.nn.functional as F
@@ -193,6 +194,10 @@ def test_calls_the_decode_kernel_leaves_to_sdpa():
     same_as_sdpa(q, k.clone().requires_grad_(True), v)
     wide = torch.randn(2, 2, 64, 132, device="cuda").bfloat16()[..., 2:130]     # rows that are not 16-byte aligned
     same_as_sdpa(q, wide, v)
+    assert decode_attn(q, k, v, None, torch.tensor(0.1)) is None                # a scale that is a tensor: SDPA's to take or to refuse
+    with pytest.raises(TypeError):
+        fn(None, q, k, v, scaling=torch.tensor([0.1]))
+    assert torch.equal(decode_attn(q, k, v, None, np.float32(0.125)), decode_attn(q, k, v, None, 0.125))
     with torch.autocast("cuda", dtype=torch.float16):
         assert decode_attn(q, k, v) is None and fn(None, q, k, v)[0].dtype == torch.float16
     batched = torch.vmap(lambda a, b, c: fn(None, a, b, c)[0])(q[None], k[None], v[None])
