@@ -569,6 +569,7 @@ int intra_b200_fwd_image_lse(const void* q, const void* k, const void* v, void* 
 const char* intra_b200_strerror(int status) {
   switch (status) {
     case INTRA_OK: return "ok";
+    case INTRA_NEED_SCRATCH: return "the scratch buffer is too small: call again with the bytes stored in *scratch_needed";
     case INTRA_ERR_BAD_ARG: return "bad argument: null pointer, non-positive size, heads not divisible, or softmax scale not positive";
     case INTRA_ERR_UNSUPPORTED: return "unsupported pattern / group_num / window / width / sequence length";
     case INTRA_ERR_ALIGNMENT: return "pointers and strides must keep every 128-element bf16 row 16-byte aligned";

@@ -31,8 +31,8 @@ def test_every_declared_symbol_is_exported(lib):
 
 def test_strerror(lib):
     assert lib.intra_b200_strerror(0) == b"ok"
-    for code in range(-6, 0):
-        assert len(lib.intra_b200_strerror(code)) > 10
+    for code in [*range(-6, 0), 1]:
+        assert len(lib.intra_b200_strerror(code)) > 10 and lib.intra_b200_strerror(code) != b"unknown status"
     assert lib.intra_b200_strerror(-99) == b"unknown status"
 
 
