@@ -186,6 +186,9 @@ int intra_b200_test_kernel_form(int family, int pattern, int S, int param, int H
  * is the attention kernel's two seconds, waited before the first warp's give-up released it. */
 int intra_b200_test_poke_status(int device, int value);
 int intra_b200_test_wait_timeout(int limit_ms, long long* waited_ns_dev, int device, void* cuda_stream);
+/* Copies 32768 bytes (`bytes`) of device memory through shared memory with bulk copies that only the attention kernel's
+ * wait for copies in flight, run when a call gives up, waits for. */
+int intra_b200_test_drain(const void* src, void* dst, int64_t bytes, int device, void* cuda_stream);
 
 /* intra_b200_fwd_llm for hosts that cannot let a library allocate device memory. It has no
  * counterpart in the reference.

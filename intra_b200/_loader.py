@@ -48,6 +48,7 @@ SIGNATURES = {
     "intra_b200_test_kernel_form": (_i, [_i, _i, _i, _i, _i, _i]),
     "intra_b200_test_poke_status": (_i, [_i, _i]),
     "intra_b200_test_wait_timeout": (_i, [_i, _vp, _i, _vp]),
+    "intra_b200_test_drain": (_i, [_vp, _vp, _i64, _i, _vp]),
 }
 
 

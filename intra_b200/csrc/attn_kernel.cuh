@@ -10,8 +10,8 @@
 //
 // Abort protocol of every kernel in this directory: all waits are bounded (ptx::mbar_wait). A wait
 // that runs out raises the CTA's shared abort flag with the id of the wait site; every other role
-// sees the flag in its own next wait and leaves its loop; the CTA then lets tensor-core work in flight
-// finish, frees its tensor memory and records STATUS_WAIT_BASE + id in the status word with an
+// sees the flag in its own next wait and leaves its loop; the CTA then lets tensor-core work and copies in
+// flight finish, frees its tensor memory and records STATUS_WAIT_BASE + id in the status word with an
 // atomicCAS from 0, so the word keeps the first failure until the host resets it. Kernels never read
 // the word: a recorded failure does not turn later launches into no-ops.
 #pragma once

@@ -589,7 +589,10 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem, 512);
   }
-  if (tid == 0 && abort_flag != 0) atomicCAS(p.f.status, 0, STATUS_WAIT_BASE + abort_flag);
+  if (tid == 0 && abort_flag != 0) {
+    ptx::drain_copies(bars, S_FULL);                       // the Q, K and V tiles that were requested before the give-up
+    atomicCAS(p.f.status, 0, STATUS_WAIT_BASE + abort_flag);
+  }
 }
 
 }  // namespace intra

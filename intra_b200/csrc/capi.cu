@@ -755,6 +755,18 @@ int intra_b200_test_wait_timeout(int limit_ms, long long* waited_ns_dev, int dev
   return e == cudaSuccess ? INTRA_OK : cuda_fail(e);
 }
 
+int intra_b200_test_drain(const void* src, void* dst, int64_t bytes, int device, void* cuda_stream) {
+  if (!src || !dst || bytes != DRAIN_BYTES) return INTRA_ERR_BAD_ARG;
+  if (!aligned16(src) || !aligned16(dst)) return INTRA_ERR_ALIGNMENT;
+  DeviceGuard guard(device);
+  if (!guard.ok) return cuda_fail(cudaGetLastError());
+  int rc = ensure_device(device);
+  if (rc != INTRA_OK) return rc;
+  drain_selftest_kernel<<<1, 128, 0, static_cast<cudaStream_t>(cuda_stream)>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst));
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? INTRA_OK : cuda_fail(e);
+}
+
 int intra_b200_test_tma_rows(const void* q, const void* k, const void* v, int B, int S, int H, int Hkv,
                              const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],
                              int family, int pattern, int param, int32_t* q_got_dev, int32_t* k_got_dev,

@@ -61,7 +61,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(smem_u32(bar), parity, abort_flag, limit_ms);
 }
-// The same by shared-memory address, and with the site's code left in *abort_flag when this wait is the one that
+// For a CTA that gives up: waits until the bulk copies counted on the `n` barriers from `bars` on have landed, so that
+// none is under way to its shared memory when it ends. The current phase of a barrier ends with its copy, whatever
+// its parity; without one the wait runs out.
+__device__ __forceinline__ void drain_copies(uint64_t* bars, int n) {
+#pragma unroll 1
+  for (int i = 0; i < 2 * n; ++i) {
+    int gave_up = 0;
+    mbar_wait(bars + (i >> 1), i & 1, &gave_up, 5);
+  }
+}
+// mbar_wait by shared-memory address, and with the site's code left in *abort_flag when this wait is the one that
 // runs out. Written for little code: the loop that waits is a handful of instructions, the clock is only
 // read every 64 tries.
 __device__ __forceinline__ bool mbar_wait_at(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {

@@ -2,7 +2,7 @@
 // through the same tile layout, descriptors and TMEM paths as the attention kernel; a kernel that
 // enumerates the (query, key) pairs the device-side index maps visit; a kernel that fetches every
 // query and key tile of a problem through the attention kernel's own TMA code and reports which token
-// rows arrived; and a kernel whose wait is never satisfied, to exercise the abort protocol.
+// rows arrived; and, for the abort protocol, a kernel whose wait is never satisfied and one that drains its copies.
 #pragma once
 #include "attn_kernel.cuh"
 #include "attn_kernel_rows.cuh"
@@ -223,6 +223,30 @@ __global__ void __launch_bounds__(64, 1) abort_selftest_kernel(int limit_ms, int
     ptx::tmem_dealloc(tmem, 32);
   }
   if (tid == 0 && abort_flag != 0) atomicCAS(status, 0, STATUS_WAIT_BASE + abort_flag);
+}
+
+// Copies DRAIN_BYTES from src through shared memory to dst in two bulk copies that nothing but drain_copies waits for:
+// one on a barrier in its second phase, one on a barrier in its first, an idle barrier between them.
+constexpr int DRAIN_BYTES = 32768;
+__global__ void __launch_bounds__(128, 1) drain_selftest_kernel(const uint4* src, uint4* dst) {
+  __shared__ __align__(128) uint4 room[DRAIN_BYTES / 16];
+  __shared__ uint64_t bars[3];
+  constexpr int HALF = DRAIN_BYTES / 32;
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    for (int i = 0; i < 3; ++i) ptx::mbar_init(&bars[i], 1);
+    ptx::fence_mbar_init();
+    ptx::mbar_arrive(&bars[0]);
+    for (int half = 0; half < 2; ++half) {
+      const uint32_t bar = ptx::smem_u32(&bars[2 * half]);
+      ptx::mbar_expect_tx_at(bar, DRAIN_BYTES / 2);
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                   :: "r"(ptx::smem_u32(room + half * HALF)), "l"(src + half * HALF), "r"(DRAIN_BYTES / 2), "r"(bar) : "memory");
+    }
+    ptx::drain_copies(bars, 3);
+  }
+  __syncthreads();
+  for (int i = tid; i < DRAIN_BYTES / 16; i += 128) dst[i] = room[i];
 }
 
 }  // namespace intra

@@ -273,6 +273,16 @@ def test_bounded_wait_gives_up_and_reports(lib):
     _util.check_against_oracle(out, q, k, v, oracle.llm_window_mask(512, 576))
 
 
+def test_a_cta_that_gives_up_waits_for_its_copies(lib):
+    """Bulk copies that nothing else waits for have landed when the wait for copies in flight returns, on barriers in
+    either phase; a barrier without a copy holds it up for milliseconds only."""
+    src = torch.randint(256, (32768,), dtype=torch.uint8, device="cuda")
+    dst = torch.zeros_like(src)
+    assert lib.intra_b200_test_drain(src.data_ptr(), dst.data_ptr(), 32768, 0, torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(src, dst)
+    assert lib.intra_b200_test_drain(src.data_ptr(), dst.data_ptr(), 100, 0, None) == -1
+
+
 @pytest.mark.parametrize("family,pattern,S,param", [
     ("llm", "scatter", 1111, 5), ("llm", "gather1", 777, 4), ("llm", "gather1", 1000, 8),
     ("llm", "window", 130, 64), ("llm", "window", 129, 200), ("llm", "scatter", 1, 1),
