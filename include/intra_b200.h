@@ -179,6 +179,12 @@ int intra_b200_test_force_path(int no_tma, int softmax_split);
  * reference's MASK_SWITCH / launch-template choice (flash_fwd_launch_template.h:401-565). */
 int intra_b200_test_kernel_form(int family, int pattern, int S, int param, int H, int Hkv);
 
+/* Test hook, host arithmetic only: how the launcher deals a problem's items to n_cta CTAs (row_gathers != 0: as for
+ * tensors no TMA box describes): the waves the items run in, and the load of the longest CTA and of all, in tenths of a
+ * key tile with seven tenths per item. */
+int intra_b200_test_deal(int family, int pattern, int S, int param, int B, int H, int Hkv, int row_gathers, int n_cta,
+                         int* n_waves, int64_t* longest, int64_t* total);
+
 /* Test hooks for the failure path (the reference has none). _poke_status synchronises the device and
  * overwrites its status word from the host. _wait_timeout launches a two-warp kernel in which one
  * warp's wait is never satisfied and runs out after limit_ms (1..1000); it returns normally, leaves

@@ -310,38 +310,73 @@ int pick_form(const Problem& prob, int row_pairs, int split_kv) {
   return form;
 }
 
-int plan_launch(const FwdParams& p, DualParams* d, int* split) {
-  d->f = p;
-  d->split_kv = p.prob.kind == KIND_IMG_GATHER0 ? 1 : 0;
-  d->row_pairs = (d->split_kv || (p.H / p.Hkv) % 2 != 0) ? 1 : 0;
-  d->n_pair_tiles = n_pair_tiles(p.prob, d->row_pairs);
-  d->heads_per_item = d->row_pairs ? p.H : p.H / 2;
-  const int64_t items = int64_t(d->n_pair_tiles) * p.B * d->heads_per_item;
+// Is the static deal of `n_waves` waves of `combos` (batch, head) combinations each within 15 % of the average load on its
+// longest CTA? Waves of less than a few rounds of the CTAs, heaviest items first and last in turn, do not fill their
+// ends: dense causal attention (one group) with 24 heads, 30 items a wave, is 36 % out. Measured where that matters, time
+// with waves over time without: 0.91-1.00 up to 14 % out of balance, 0.97-1.01 at 17-19 %, 1.18 at 28 % and 36 %.
+bool waves_balance(const Problem& prob, int row_pairs, int combos, int n_waves, int n_cta) {
+  constexpr int MAX_CTA = 256;
+  if (n_cta > MAX_CTA) return false;
+  int64_t load[MAX_CTA] = {}, total = 0;
+  const int step = row_pairs ? 2 : 1, levels = ceil_div(prob.tiles_m, step);
+  int cta = 0, dir = 1;                  // dual_item_index, one item after the other
+  for (int w = 0; w < n_waves; ++w)
+    for (int l = 0; l < levels; ++l) {
+      const int level = (n_waves - 1 - w) & 1 ? levels - 1 - l : l;
+      const int weight = 10 * (prob.tiles_m - step * level) + 7;       // key tiles, and 0.7 of one for the item's ends
+      for (int i = 0; i < prob.G * combos; ++i) {
+        load[cta] += weight;
+        total += weight;
+        const int next = cta + dir;
+        if (next < 0 || next >= n_cta) dir = -dir; else cta = next;
+      }
+    }
+  int64_t longest = 0;
+  for (int i = 0; i < n_cta; ++i) longest = load[i] > longest ? load[i] : longest;
+  return longest * n_cta * 100 <= total * 115;
+}
+
+// Pair tiles, items and the order they are numbered in.
+int plan_items_order(const Problem& prob, int B, int H, int Hkv, int use_tma, int n_cta, DualParams* d) {
+  d->split_kv = prob.kind == KIND_IMG_GATHER0 ? 1 : 0;
+  d->row_pairs = (d->split_kv || (H / Hkv) % 2 != 0) ? 1 : 0;
+  d->n_pair_tiles = n_pair_tiles(prob, d->row_pairs);
+  d->heads_per_item = d->row_pairs ? H : H / 2;
+  const int64_t items = int64_t(d->n_pair_tiles) * B * d->heads_per_item;
   if (items <= 0 || items > 0x7fffffffLL) return INTRA_ERR_UNSUPPORTED;
   d->n_items = static_cast<int>(items);
   // All (batch, head) combinations run through the pair tiles, heaviest first, together - unless a grouped pattern's
-  // K and V are larger than the L2: every level of row tiles then reads all of them from HBM again (7.0 GB per
-  // launch at 65536 tokens and 8 KV heads, 1.3 GB compulsory). One KV head at a time, its K and V stay. GPU time of
-  // Scatter G=8, 32/8 heads, 65536 tokens 3431 -> 3178 us (back to back under the power cap 3800 -> 3505), of which
-  // waves that all run from heavy to light, 6 % out of balance, gave half (3467 -> 3325; 46000 tokens 1729 -> 1632,
-  // 32768 (134 MB) 892 -> 874, 32/32 heads 32768 1058 -> 966). Smaller ones only lose balance: G=2 23000 tokens
-  // (94 MB) 1585 -> 1687.
+  // K and V are larger than the L2: every level of row tiles then reads all of them from HBM again. One KV head at a
+  // time, its K and V stay. GPU time of one launch without / with waves (idle GPU, one B200): G=8, 32/8 heads, 65536 tokens
+  // 3533 / 3233 us, 46000 1747 / 1619, 32768 894 / 844; G=2 32768 3224 / 3135; 32/32 heads 32768 1088 / 934, 9000 112 /
+  // 107, 8192 at G=2 244 / 244. Not for groups of one level, which read nothing twice (1.9 % slower at worst), nor for
+  // the row gathers, where their loads bound the items (G=7, 32/32 heads, 16384 tokens 786 / 982 us).
   constexpr int64_t L2_BYTES = 126ll << 20;
-  const bool grouped = p.prob.kind == KIND_LLM_SCATTER || p.prob.kind == KIND_LLM_GATHER1;
-  const int64_t kv_bytes = int64_t(p.B) * p.prob.S * p.Hkv * (2 * HEAD_DIM * 2);
-  const int per_kv_head = d->row_pairs ? p.H / p.Hkv : p.H / p.Hkv / 2;
-  const int combos = grouped && kv_bytes > L2_BYTES ? per_kv_head : p.B * d->heads_per_item;
+  const bool grouped = prob.kind == KIND_LLM_SCATTER || prob.kind == KIND_LLM_GATHER1;
+  const int64_t kv_bytes = int64_t(B) * prob.S * Hkv * (2 * HEAD_DIM * 2);
+  const int all = B * d->heads_per_item, per_kv_head = d->row_pairs ? H / Hkv : H / Hkv / 2;
+  const bool waves = use_tma && grouped && kv_bytes > L2_BYTES && d->n_pair_tiles > prob.G &&
+                     (int64_t(d->n_pair_tiles) * per_kv_head >= 3 * n_cta ||
+                      waves_balance(prob, d->row_pairs, per_kv_head, all / per_kv_head, n_cta));
+  const int combos = waves ? per_kv_head : all;
   d->by_wave = fast_div(d->n_pair_tiles * combos);
   d->by_tile = fast_div(combos);
-  d->last_wave = p.B * d->heads_per_item / combos - 1;
+  d->last_wave = all / combos - 1;
   d->by_heads = fast_div(d->heads_per_item);
-  d->by_rep = fast_div(p.H / p.Hkv);
-  d->wide_stores = (reinterpret_cast<uintptr_t>(p.o) % 32 == 0 && p.os.sb % 16 == 0 && p.os.ss % 16 == 0 && p.os.sh % 16 == 0) ? 1 : 0;
+  d->by_rep = fast_div(H / Hkv);
+  return INTRA_OK;
+}
+
+int plan_launch(const FwdParams& p, int sm_count, DualParams* d, int* split) {
+  d->f = p;
   d->use_tma = !g_force_no_tma.load() && tma_supported(p.prob) &&
                build_maps(p.prob, p.q, p.qs, p.H, p.B, 0, &d->maps) && build_maps(p.prob, p.k, p.ks, p.Hkv, p.B, 1, &d->maps) &&
                build_maps(p.prob, p.v, p.vs, p.Hkv, p.B, 2, &d->maps) &&
                (p.prob.kind == KIND_IMG_SCATTER || p.prob.kind == KIND_IMG_GATHER0 ||
                 build_maps(p.prob, p.o, p.os, p.H, p.B, 3, &d->maps));
+  const int rc = plan_items_order(p.prob, p.B, p.H, p.Hkv, d->use_tma, sm_count, d);
+  if (rc != INTRA_OK) return rc;
+  d->wide_stores = (reinterpret_cast<uintptr_t>(p.o) % 32 == 0 && p.os.sb % 16 == 0 && p.os.ss % 16 == 0 && p.os.sh % 16 == 0) ? 1 : 0;
   *split = d->use_tma ? 0 : pick_form(p.prob, d->row_pairs, d->split_kv);
   return INTRA_OK;
 }
@@ -367,7 +402,7 @@ int launch_fwd(const void* q, const void* k, const void* v, void* out, int B, in
   p.lse = lse;
   DualParams d;
   int split = 0;
-  int rc = plan_launch(p, &d, &split);
+  int rc = plan_launch(p, sm_count, &d, &split);
   if (rc != INTRA_OK) return rc;
   const int grid = d.n_items < sm_count ? d.n_items : sm_count;     // persistent: one CTA per SM
 #define INTRA_LAUNCH_ROWS(KIND) \
@@ -726,6 +761,30 @@ int intra_b200_test_kernel_form(int family, int pattern, int S, int param, int H
   return pick_form(prob, row_pairs, split_kv);
 }
 
+int intra_b200_test_deal(int family, int pattern, int S, int param, int B, int H, int Hkv, int row_gathers, int n_cta, int* n_waves,
+                         int64_t* longest, int64_t* total) {
+  if (B <= 0 || S <= 0 || H <= 0 || Hkv <= 0 || H % Hkv != 0 || n_cta <= 0 || !n_waves || !longest || !total) return INTRA_ERR_BAD_ARG;
+  Problem prob;
+  int rc = problem_from(family, pattern, S, param, &prob);
+  if (rc != INTRA_OK) return rc;
+  DualParams d;
+  rc = plan_items_order(prob, B, H, Hkv, !row_gathers && tma_supported(prob), n_cta, &d);
+  if (rc != INTRA_OK) return rc;
+  *n_waves = d.last_wave + 1;
+  *longest = *total = 0;
+  for (int cta = 0; cta < n_cta; ++cta) {
+    int64_t load = 0;
+    for (int seq = 0; int64_t(seq) * n_cta < d.n_items; ++seq) {
+      const int item = dual_item_index(seq, cta, n_cta);
+      const int n_kv = item < d.n_items ? dual_decode(d, prob, item).pt.kv.n_kv_tiles : 0;
+      load += n_kv > 0 ? 10 * n_kv + 7 : 0;
+    }
+    *total += load;
+    *longest = load > *longest ? load : *longest;
+  }
+  return INTRA_OK;
+}
+
 int intra_b200_test_force_path(int no_tma, int softmax_split) {
   if (softmax_split != 0 && softmax_split != 1 && softmax_split != 2 && softmax_split != 4) return INTRA_ERR_BAD_ARG;
   g_force_no_tma.store(no_tma ? 1 : 0);
@@ -800,7 +859,7 @@ int intra_b200_test_tma_rows(const void* q, const void* k, const void* v, int B,
   DualParams d;
   int split = 0;
   const int forced = g_force_no_tma.exchange(0);           // the maps are wanted whatever the override says
-  rc = plan_launch(p, &d, &split);
+  rc = plan_launch(p, g_dev[device].sm_count, &d, &split);
   g_force_no_tma.store(forced);
   if (rc != INTRA_OK) return rc;
   if (!d.use_tma) return INTRA_ERR_UNSUPPORTED;

@@ -122,3 +122,32 @@ def test_image_widths_whose_square_wraps_are_refused(lib):
     nt, nkv = ctypes.c_int64(0), ctypes.c_int64(0)
     for pattern in (0, 4):
         assert lib.intra_b200_tile_counts(1, pattern, 512, 65536, ctypes.byref(nt), ctypes.byref(nkv)) == -2
+
+
+def _deal(lib, pattern, S, G, B, H, Hkv, row_gathers=0):
+    waves, longest, total = ctypes.c_int(0), ctypes.c_int64(0), ctypes.c_int64(0)
+    assert lib.intra_b200_test_deal(0, _util.PATTERN_ID[("llm", pattern)], S, G, B, H, Hkv, row_gathers, 148, ctypes.byref(waves),
+                                    ctypes.byref(longest), ctypes.byref(total)) == 0
+    return waves.value, longest.value * 148 / total.value
+
+
+def test_waves_of_kv_heads_keep_the_ctas_balanced(lib):
+    """K and V beyond the L2 run one KV head at a time, where that leaves the longest CTA within 15 % of the average (two
+    more for groups of two lengths, which the rule does not tell apart)."""
+    taken = {}
+    for H, Hkv in ((32, 8), (32, 32), (24, 24), (64, 64), (64, 8), (28, 4), (16, 16), (4, 1)):
+        for G in (1, 2, 3, 8, 64):
+            for S in (464, 1000, 2532, 5330, 7467, 9013, 16384, 32768, 65536):
+                for B in (1, 2, 4, 16):
+                    waves, out = _deal(lib, "scatter", S, G, B, H, Hkv)
+                    assert waves in (1, B * Hkv) and (waves == 1 or B * S * Hkv * 512 > 126 << 20)
+                    assert waves == 1 or out <= 1.17, (S, G, B, H, Hkv, out)
+                    taken[S, G, B, H, Hkv] = waves > 1
+    assert taken[65536, 8, 1, 32, 8] and taken[32768, 2, 1, 32, 8] and taken[32768, 8, 1, 32, 32]     # measured gains
+    assert not taken[7467, 1, 2, 24, 24] and not taken[464, 1, 16, 64, 64]                            # measured losses
+    assert not taken[1000, 8, 16, 32, 32]                                                             # one level: nothing is read twice
+
+
+def test_row_gathers_run_without_waves(lib):
+    assert _deal(lib, "gather1", 16384, 7, 1, 32, 32)[0] == 1          # no TMA boxes for groups of 7
+    assert _deal(lib, "scatter", 65536, 8, 1, 32, 8, row_gathers=1)[0] == 1
