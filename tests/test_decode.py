@@ -67,7 +67,7 @@ def _reference(q, k, v, mask, scale):
     (1, 4, 1, 63, "bhsd", "random"), (2, 32, 8, 64, "sliced", None), (3, 32, 8, 65, "batch1", "shared"),
     (1, 32, 8, 1023, "bhsd", None), (1, 32, 8, 1024, "bhsd", None), (1, 32, 8, 3001, "bshd", None),   # clusters of 8 / 16
     (1, 32, 8, 8191, "bhsd", None), (1, 4, 1, 40000, "sliced", None),                                 # several clusters
-    (16, 32, 8, 2100, "bhsd", "left-padded"), (20, 32, 32, 300, "bhsd", None), (300, 4, 1, 40, "bhsd", "one-key"),
+    (16, 32, 8, 2100, "bhsd", "left-padded"), (20, 32, 32, 300, "bhsd", "random"), (3, 32, 32, 70, "bhsd", None), (300, 4, 1, 40, "bhsd", "one-key"),
     (2, 9, 1, 500, "bhsd", "random"), (2, 36, 2, 77, "bhsd", "strided"), (1, 64, 2, 5000, "bshd", "longer"),   # 9, 18, 32 heads per KV head
     (40, 16, 8, 2500, "bhsd", "random")])
 def test_decode_kernel_vs_fp64(B, H, Hkv, S, layout, mask):
@@ -143,6 +143,36 @@ def test_decode_kernel_under_capture_and_on_other_streams():
     graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,S,kernel", [
+    (1, 8, 900, True), (16, 32, 100, True), (1, 32, 1710, True), (1, 32, 6100, True),      # up to 28 MB; 32 heads: up to 100 MB
+    (1, 32, 6110, False), (16, 32, 110, False), (20, 32, 300, False), (32, 32, 20, False)])
+def test_multi_head_caches_go_where_they_are_quicker(B, H, S, kernel):
+    q, k, v = _inputs(B, H, H, S)
+    fn = make_intra_attention()
+    sdpa = F.scaled_dot_product_attention(q, k, v).transpose(1, 2)
+    out, mine = fn(None, q, k, v)[0], decode_attn(q, k, v)
+    assert (mine is not None) == kernel and torch.equal(out, mine if kernel else sdpa)
+    masked = decode_attn(q, k, v, torch.ones(B, 1, 1, S, dtype=torch.bool, device="cuda"))
+    assert float((masked.float() - sdpa.float()).abs().max()) <= 1.6e-2
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        replayed = fn(None, q, k, v)[0]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(replayed, out)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,S,kernel", [(128, 32, False), (128, 33, True), (64, 32, True)])
+def test_masked_multi_head_caches_go_where_they_are_quicker(B, S, kernel):
+    q, k, v = _inputs(B, 32, 32, S)
+    m = _mask("left-padded", B, S)
+    out, mine = make_intra_attention()(None, q, k, v, m)[0], decode_attn(q, k, v, m)
+    assert (mine is not None) == kernel
+    assert torch.equal(out, mine if kernel else F.scaled_dot_product_attention(q, k, v, attn_mask=m).transpose(1, 2))
 
 
 @pytest.mark.gpu
