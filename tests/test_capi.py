@@ -110,13 +110,22 @@ def test_helper_entry_points_reject_bad_arguments(lib):
 
 
 def test_launcher_picks_the_kernel_form_by_item_length(lib):
-    """Host arithmetic only: long items that share their key tiles go to the row-owner form, short ones
-    (window: 5 key tiles, Gather-0: 7, S=4096) to the 4-way column split; a forced form is honoured, with
-    the 2-way split standing in for the row-owner form on split key lists."""
+    """Host arithmetic only, the row-gather kernel's form for the problems that reach it - ragged Gather-1, image widths
+    without TMA boxes, and any shape on expanded tensors: long items that share their key tiles go to the row-owner
+    form, short ones (window: 5 key tiles, Gather-0: 7, S=4096) to the 4-way column split; a forced form is honoured,
+    with the 2-way split standing in for the row-owner form on split key lists."""
     form = lib.intra_b200_test_kernel_form
     LLM, IMG = 0, 1
     SCATTER, GATHER1, WINDOW, GATHER0 = 0, 1, 4, 4
-    assert form(LLM, SCATTER, 4096, 8, 32, 8) == 4            # 2.5 key tiles per item
+    assert form(LLM, GATHER1, 16385, 8, 32, 8) == 1           # 8.6 key tiles per item
+    assert form(LLM, GATHER1, 16384, 7, 32, 32) == 1
+    assert form(LLM, GATHER1, 5000, 8, 32, 8) == 4
+    assert form(IMG, SCATTER, 512 + 48 * 48, 48, 24, 24) == 4     # 7
+    assert form(IMG, SCATTER, 512 + 96 * 96, 96, 24, 24) == 1     # 13
+    assert form(IMG, GATHER0, 512 + 40 * 40, 40, 24, 24) == 4
+    # expanded tensors
+    assert form(LLM, WINDOW, 16384, 1000, 32, 8) == 1
+    assert form(LLM, SCATTER, 4096, 8, 32, 8) == 4            # 2.5
     assert form(LLM, GATHER1, 16384, 8, 32, 8) == 1           # 8.5
     assert form(LLM, WINDOW, 16384, 576, 32, 8) == 4
     assert form(LLM, SCATTER, 32768, 2, 32, 8) == 1

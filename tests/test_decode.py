@@ -65,7 +65,10 @@ def _reference(q, k, v, mask, scale):
 @pytest.mark.parametrize("B,H,Hkv,S,layout,mask", [
     (1, 32, 8, 1, "bhsd", None), (1, 32, 8, 15, "bhsd", None), (1, 32, 8, 17, "bshd", None),       # ends of a 16-key block
     (1, 4, 1, 63, "bhsd", "random"), (2, 32, 8, 64, "sliced", None), (3, 32, 8, 65, "batch1", "shared"),
-    (1, 32, 8, 1023, "bhsd", None), (1, 32, 8, 1024, "bhsd", None), (1, 32, 8, 3001, "bshd", None),   # clusters of 8 / 16
+    (1, 32, 8, 1008, "bhsd", None), (1, 32, 8, 1009, "bhsd", None), (1, 32, 8, 3001, "bshd", None),   # clusters of 8, of 16
+    (1, 32, 8, 8176, "bhsd", None), (5, 32, 8, 300, "bhsd", "random"),                               # the last of 16; of 4
+    (16, 16, 8, 8192, "batch1", "left-padded"),               # 2 CTAs a unit would do, 4 are needed: 128 blocks each, all they can list
+    (8, 8, 8, 16384, "batch1", "random"), (8, 16, 8, 16400, "batch1", "random"),    # 8 are full; one block more takes a second cluster
     (1, 32, 8, 8191, "bhsd", None), (1, 4, 1, 40000, "sliced", None),                                 # several clusters
     (16, 32, 8, 2100, "bhsd", "left-padded"), (20, 32, 32, 300, "bhsd", "random"), (3, 32, 32, 70, "bhsd", None), (300, 4, 1, 40, "bhsd", "one-key"),
     (2, 9, 1, 500, "bhsd", "random"), (2, 36, 2, 77, "bhsd", "strided"), (1, 64, 2, 5000, "bshd", "longer"),   # 9, 18, 32 heads per KV head

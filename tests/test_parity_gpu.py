@@ -487,12 +487,16 @@ def _launcher_choice_restored(lib):
     assert lib.intra_b200_test_force_path(0, 0) == 0
 
 
-@pytest.mark.parametrize("no_tma,split", [(0, 1), (0, 2), (0, 4), (1, 0), (1, 1), (1, 2), (1, 4)],
-                         ids=["row-owner", "split2", "split4", "no-tma", "no-tma-row-owner", "no-tma-split2", "no-tma-split4"])
+# The kernel for TMA shapes, which has one form, and the row-gather kernel in the form the launcher picks and in each of
+# its three (on split key lists, Gather-0's, the row-owner form is the 2-way split).
+KERNEL_PATHS = pytest.mark.parametrize("no_tma,split", [(0, 0), (1, 0), (1, 1), (1, 2), (1, 4)],
+                                       ids=["tma", "row-gathers", "row-owner", "split2", "split4"])
+
+
+@KERNEL_PATHS
 def test_forced_kernel_paths(lib, _launcher_choice_restored, no_tma, split):
-    """Every kernel variant the launcher can choose, forced through the library's test hook: the
-    row-owner form and both softmax column splits for every pattern, including the combinations its
-    heuristic never picks, and the cp.async row gathers where TMA boxes would have been used."""
+    """Every kernel variant, forced through the library's test hook, on every pattern, including the
+    combinations the launcher never picks."""
     from intra_b200 import intra_image_attn, intra_llm_attn
     assert lib.intra_b200_test_force_path(no_tma, split) == 0
     with torch.no_grad():
@@ -508,14 +512,14 @@ def test_forced_kernel_paths(lib, _launcher_choice_restored, no_tma, split):
             assert float((lse - oracle.masked_lse(q, k, mask)).abs().max()) <= LSE_ATOL, (family, pattern)
 
 
-@pytest.mark.parametrize("split", [1, 2, 4], ids=["row-owner", "split2", "split4"])
-def test_items_of_one_key_tile_back_to_back(lib, _launcher_choice_restored, split):
+@KERNEL_PATHS
+def test_items_of_one_key_tile_back_to_back(lib, _launcher_choice_restored, no_tma, split):
     """Scatter with 128-token groups: every item of every CTA has a single key tile, so nothing but the
-    hand-offs between the softmax warps, the MMA warps and the epilogue warps paces the pipeline from
+    hand-offs between the loading, softmax, MMA and (TMA shapes) epilogue warps paces the pipeline from
     item to item (the case in which a role can run furthest ahead of another). Output and log-sum-exp
     against the oracle, and no bounded wait gave up."""
     from intra_b200 import intra_llm_attn
-    assert lib.intra_b200_test_force_path(0, split) == 0
+    assert lib.intra_b200_test_force_path(no_tma, split) == 0
     S, G = 2048, 16
     q, k, v = oracle.make_inputs(4, S, 16, 8, seed=41, device="cuda")
     mask = torch.from_numpy(oracle.build_mask("llm", "scatter", S, group_num=G)).cuda()

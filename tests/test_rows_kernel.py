@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
     ("scatter", 1, 2047, 4, 2, 8), ("scatter", 2, 2049, 3, 3, 8), ("scatter", 1, 1031, 4, 4, 7),   # groups of two lengths
     ("scatter", 1, 300, 2, 1, 299), ("scatter", 1, 128 * 3 + 1, 2, 1, 3),                          # one- and two-token groups; a tile of one row
     ("scatter", 24, 256, 32, 16, 2),          # 768 items of one key tile: a batch of the planner is full on some CTAs
-    ("scatter", 80, 200, 32, 32, 8),          # 10240 items: several batches per CTA, the last one partly filled
+    ("scatter", 80, 200, 32, 32, 8),          # 20480 items: several batches per CTA, the last one partly filled
     ("gather1", 1, 4096, 2, 1, 64), ("gather1", 1, 128 * 128, 2, 2, 128),   # 32-row output boxes inside one segment
     ("gather1", 1, 64 * 9, 4, 2, 8), ("gather1", 3, 16 * 33, 4, 4, 4),
     ("window", 1, 1, 2, 1, 576), ("window", 2, 33, 2, 2, 64), ("window", 1, 4129, 4, 1, 1000), ("window", 1, 575, 3, 1, 65)])
