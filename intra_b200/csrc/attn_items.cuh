@@ -12,7 +12,7 @@ struct DualParams {
   int heads_per_item;   // row_pairs ? H : H / 2  (number of items per pair tile and batch)
   int n_items;          // n_pair_tiles * B * heads_per_item
   int last_wave;        // waves alternate between heaviest and lightest first; the last one ends with the lightest
-  // Items are numbered wave by wave (plan_launch), within a wave pair tile by pair tile: divisors items per wave,
+  // Items are numbered wave by wave (plan_items_order), within a wave pair tile by pair tile: divisors items per wave,
   // (batch, head) combinations per wave, heads_per_item, H / Hkv.
   FastDiv by_wave, by_tile, by_heads, by_rep;
   int split_kv;         // the two sub-tiles keep their own key lists (Gather-0): K / V buffer s belongs to sub-tile s

@@ -1,5 +1,5 @@
-// Definitions shared by the attention kernel (attn_kernel_dual.cuh) and the device self-tests
-// (selftest.cuh): tile geometry, the parameter block, the shared-memory tile layout and the two
+// Definitions shared by the attention kernels (attn_kernel_rows.cuh for TMA shapes, attn_kernel_dual.cuh for row
+// gathers, decode_kernel.cuh for one token) and the device self-tests (selftest.cuh): tile geometry, the parameter block, the shared-memory tile layout and the two
 // tensor-core contractions of flash attention on sm_100a,
 //
 //   S = Q K^T    both operands 128-byte-swizzled shared-memory tiles, accumulator in tensor memory

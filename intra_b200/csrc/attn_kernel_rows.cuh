@@ -394,7 +394,8 @@ __global__ void __launch_bounds__(RowsCfg::THREADS, 1) intra_fwd_rows_kernel(con
           // A warp's 32 rows leave as two bulk stores of 64 columns each through its staging buffer (128-byte swizzle).
           // Stored by their threads, 32 bytes to 32 lines per instruction, they would hold up the sets' barrier
           // traffic behind them: GPU time of Scatter at S = 4096 30.2 -> 28.7 us, window at 16384 155.4 -> 151.2.
-          // The image patterns' strided views have no such boxes; their rows are stored by their threads.
+          // The image patterns' rows are stored by their threads: image Scatter's view has traversal strides, and for
+          // Gather-0 there is no output view.
           const int w = warp & 3;
           int c1 = sl.q[sx].c1, c2 = sl.q[sx].c2;          // the query tile's place, this warp's rows on
           if (KIND == KIND_LLM_SCATTER) c2 += OUT_ROWS * w;

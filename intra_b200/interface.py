@@ -249,47 +249,35 @@ def intra_image_attn(q, k, v, pattern="scatter", width=64, softmax_scale=None, *
     return _image(q, k, v, 1, 2, pattern, width, softmax_scale, strict, return_lse, out)
 
 
-def _one_head_each(units, S, masked):
-    """Does the decode kernel take caches of S keys with as many KV heads as query heads (`units` in the batch)? With one
-    query row per KV head it has nothing to reuse; against the kernels of SDPA (one B200, us):
-    * without a mask its GPU time is 0.9-1.7 times SDPA's over 8-8192 units of 17-24000 keys, except where its 8 CTAs per
-      unit fill the chip (32 units, K and V of 28 / 64 / 100 MB: 8.1 / 14.1 / 18.7 against 8.4 / 15.3 / 19.9). But its way
-      to the launch is shorter, which decides calls of up to 28 MB: 12.9 a call against 15.5-19.4 (replayed from a CUDA
-      graph, where that does not count, such calls take 4-13 against 3-12). At 1024 units the GPU takes longer than that:
-      16.8-18.6 a call against 15.8-17.0;
-    * with a mask it is quicker, but for the shortest caches of many units: up to 32 keys of 4096 units a call takes 64
-      against 59 (2048 units: 33 against 39).
-    The choice goes by sizes alone: a call that is captured runs what its warm-up ran."""
-    if masked:
-        return S > 32 or units < 4096
-    nbytes = units * S * 512                         # K and V
-    return (units <= 512 and nbytes <= 28e6) or (28 <= units <= 37 and nbytes <= 100e6)
-
-
 def decode_attn(q, k, v, mask=None, softmax_scale=None):
     """Dense attention of one token per sequence over its cache: q (B, H, 1, 128), k and v
     (B, Hkv, S, 128), `mask` None or bool (B or 1, 1, 1, >= S), nonzero = visible. Returns (B, 1, H, 128), or None
-    for caches of one KV head per query head on which SDPA is quicker, and
     for calls the decode kernel does not take - other types, GPUs, layouts or broadcasts, masks per
     head or additive, and everything that looks inside an operator (autograd, forward-mode, vmap, tracing,
     dispatch modes, autocast to another type) - which are the caller's to run as torch operators."""
+    # what costs least first, tracers before sizes: a call that is left to torch has paid for the questions before it
     if type(q) is not torch.Tensor or type(k) is not torch.Tensor or type(v) is not torch.Tensor:
         return None
     if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16 or not q.is_cuda:
+        return None
+    if torch.compiler.is_compiling() or _watched():
+        return None
+    if mask is not None and (type(mask) is not torch.Tensor or mask.dtype != torch.bool or mask.dim() != 4):
+        return None
+    kn = k.shape
+    if q.dim() != 4 or len(kn) != 4 or kn != v.shape:
+        return None
+    B, H, n, D = q.shape
+    Bk, Hkv, S, Dk = kn
+    if n != 1 or D != 128 or Dk != 128 or Bk != B or B == 0 or S == 0 or Hkv == 0 or H < Hkv or H % Hkv:
         return None
     if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
         return None
     if softmax_scale is not None and type(softmax_scale) is not float and not isinstance(softmax_scale, numbers.Real):
         return None
-    if (torch.compiler.is_compiling() or _watched() or q.is_neg() or k.is_neg() or v.is_neg()
-            or (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.bfloat16)):
-        return None
     dev = q.device
-    if q.dim() != 4 or k.dim() != 4 or k.shape != v.shape or k.device != dev or v.device != dev:
-        return None
-    B, H, n, D = q.shape
-    Bk, Hkv, S, Dk = k.shape
-    if n != 1 or D != 128 or Dk != 128 or Bk != B or B == 0 or S == 0 or Hkv == 0 or H < Hkv or H % Hkv:
+    if (q.is_neg() or k.is_neg() or v.is_neg() or k.device != dev or v.device != dev
+            or (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.bfloat16)):
         return None
     qs, ks, vs = q.stride(), k.stride(), v.stride()
     qp, kp, vp = q.data_ptr(), k.data_ptr(), v.data_ptr()
@@ -298,12 +286,9 @@ def decode_attn(q, k, v, mask=None, softmax_scale=None):
         return None
     mp, ms0, ms1 = None, 0, 0
     if mask is not None:
-        if (type(mask) is not torch.Tensor or mask.dtype != torch.bool or mask.dim() != 4 or mask.device != dev
-                or mask.shape[0] not in (1, B) or mask.shape[1] != 1 or mask.shape[2] != 1 or mask.shape[3] < S):
+        if mask.device != dev or mask.shape[0] not in (1, B) or mask.shape[1] != 1 or mask.shape[2] != 1 or mask.shape[3] < S:
             return None
         mp, ms0, ms1 = mask.data_ptr(), mask.stride(0) if mask.shape[0] == B else 0, mask.stride(3)
-    if H == Hkv and not _one_head_each(B * H, S, mask is not None):
-        return None
     out = q.new_empty((B, 1, H, D))
     need = ctypes.c_int64(0)
     scratch, nbytes = None, 0

@@ -6,7 +6,8 @@ layers, then two 64-aligned-window layers, repeating, with dense attention for s
 steps because the patterns are prefill-only. This module offers the same callable with the prefill
 running on the B200 kernels: query/key/value arrive as (B, H, S, D) and are handed to the kernel as
 (B, S, H, D) views without copies. The decode step is dense over the cache, as in the reference: on the
-library's decode kernel for bf16 caches with or without a padding mask, else one SDPA call.
+library's decode kernel for bf16 caches with or without a padding mask, else, and for multi-head caches that
+SDPA is quicker on, one SDPA call.
 
     from transformers import AttentionInterface
     AttentionInterface.register("intra_b200", make_intra_attention())
@@ -30,6 +31,26 @@ def layer_masktype(layer_idx: int) -> int:
     return 0 if layer_idx % 4 in (0, 1) else 4
 
 
+def _kernel_is_quicker(units, S, masked):
+    """Is the decode kernel quicker than SDPA on caches of S keys with as many KV heads as query heads, `units` of them in
+    the batch? With one query row per KV head it has nothing to reuse. Measured on one B200, us:
+    * without a mask its GPU time is 0.9-1.7 times SDPA's over 8-8192 units of 17-24000 keys, except where its 8 CTAs per
+      unit fill the chip (32 units, K and V of 28 / 64 / 100 MB: 8.1 / 14.1 / 18.7 against 8.4 / 15.3 / 19.9). But its way
+      to the launch is shorter, which decides calls of up to 44 MB: 13-14.4 a call against 15.4-19.3 (replayed from a CUDA
+      graph, where that does not count, such calls take 4-14 against 3-12). Below 24 units the kernel takes a second launch
+      from 28 MB on (20.7 a call against 19.3), and beyond 256 units its GPU time shows (512 units, 44 MB: 17.5 against
+      15.7; 1024: 16.8-18.6 against 15.8-17.0 from the shortest caches on);
+    * with a mask it is quicker, but for the shortest caches of many units: up to 32 keys of 4096 units a call takes 64
+      against 59 (2048 units: 33 against 39).
+    The choice goes by sizes alone: a call that is captured runs what its warm-up ran."""
+    if masked:
+        return S > 32 or units < 4096
+    nbytes = units * S * 512                         # K and V
+    if 28 <= units <= 37:
+        return nbytes <= 100e6
+    return units <= 512 and nbytes <= (44e6 if 24 <= units <= 256 else 28e6)
+
+
 def make_intra_attention(num_groups: int = NUM_GROUPS, back: int = WINDOW_BACK, chunk: int = WINDOW_CHUNK,
                          force_masktype=None):
     """Returns `fn(module, query, key, value, attention_mask=None, scaling=None, dropout=0.0, **kw)`
@@ -41,10 +62,11 @@ def make_intra_attention(num_groups: int = NUM_GROUPS, back: int = WINDOW_BACK, 
     def intra_attention_forward(module, query, key, value, attention_mask=None, scaling=None, dropout=0.0,
                                 **kwargs):
         if query.shape[2] == 1:          # decode step: dense over the cache, as the reference does
-            out = decode_attn(query, key, value, attention_mask, scaling)
-            if out is not None:
-                return out, None
             rep = query.shape[1] // key.shape[1]
+            if rep != 1 or _kernel_is_quicker(query.shape[0] * query.shape[1], key.shape[2], attention_mask is not None):
+                out = decode_attn(query, key, value, attention_mask, scaling)
+                if out is not None:
+                    return out, None
             k2 = key.repeat_interleave(rep, dim=1) if rep > 1 else key
             v2 = value.repeat_interleave(rep, dim=1) if rep > 1 else value
             am = attention_mask[:, :, :, : k2.shape[-2]] if attention_mask is not None else None

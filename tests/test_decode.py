@@ -149,33 +149,24 @@ def test_decode_kernel_under_capture_and_on_other_streams():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("B,H,S,kernel", [
-    (1, 8, 900, True), (16, 32, 100, True), (1, 32, 1710, True), (1, 32, 6100, True),      # up to 28 MB; 32 heads: up to 100 MB
-    (1, 32, 6110, False), (16, 32, 110, False), (20, 32, 300, False), (32, 32, 20, False)])
-def test_multi_head_caches_go_where_they_are_quicker(B, H, S, kernel):
+@pytest.mark.parametrize("B,H,S,masked,kernel", [
+    (1, 8, 900, False, True), (1, 8, 6900, False, False), (1, 24, 3500, False, True), (2, 32, 1350, False, False),
+    (1, 32, 6100, False, True), (1, 32, 6110, False, False), (16, 32, 100, False, True), (16, 32, 110, False, False),
+    (20, 32, 300, False, False), (32, 32, 20, False, False), (128, 32, 32, True, False), (128, 32, 33, True, True),
+    (64, 32, 32, True, True)])
+def test_multi_head_caches_go_where_they_are_quicker(B, H, S, masked, kernel):
     q, k, v = _inputs(B, H, H, S)
+    m = _mask("left-padded", B, S) if masked else None
     fn = make_intra_attention()
-    sdpa = F.scaled_dot_product_attention(q, k, v).transpose(1, 2)
-    out, mine = fn(None, q, k, v)[0], decode_attn(q, k, v)
-    assert (mine is not None) == kernel and torch.equal(out, mine if kernel else sdpa)
-    masked = decode_attn(q, k, v, torch.ones(B, 1, 1, S, dtype=torch.bool, device="cuda"))
-    assert float((masked.float() - sdpa.float()).abs().max()) <= 1.6e-2
+    want = decode_attn(q, k, v, m) if kernel else F.scaled_dot_product_attention(q, k, v, attn_mask=m).transpose(1, 2)
+    out = fn(None, q, k, v, m)[0]
+    assert torch.equal(out, want)
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
-        replayed = fn(None, q, k, v)[0]
+        replayed = fn(None, q, k, v, m)[0]
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(replayed, out)
-
-
-@pytest.mark.gpu
-@pytest.mark.parametrize("B,S,kernel", [(128, 32, False), (128, 33, True), (64, 32, True)])
-def test_masked_multi_head_caches_go_where_they_are_quicker(B, S, kernel):
-    q, k, v = _inputs(B, 32, 32, S)
-    m = _mask("left-padded", B, S)
-    out, mine = make_intra_attention()(None, q, k, v, m)[0], decode_attn(q, k, v, m)
-    assert (mine is not None) == kernel
-    assert torch.equal(out, mine if kernel else F.scaled_dot_product_attention(q, k, v, attn_mask=m).transpose(1, 2))
 
 
 @pytest.mark.gpu
