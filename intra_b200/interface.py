@@ -260,9 +260,9 @@ def decode_attn(q, k, v, mask=None, softmax_scale=None):
         return None
     if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16 or not q.is_cuda:
         return None
-    if torch.compiler.is_compiling() or _watched():
-        return None
     if mask is not None and (type(mask) is not torch.Tensor or mask.dtype != torch.bool or mask.dim() != 4):
+        return None
+    if torch.compiler.is_compiling() or _watched():
         return None
     kn = k.shape
     if q.dim() != 4 or len(kn) != 4 or kn != v.shape:
