@@ -44,10 +44,10 @@ if ROOT not in sys.path:
 HEAD_DIM = 128
 FALLBACK_PEAKS = {"bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0, "hbm_gbs": 6650.0}
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of each workload's dominant kernel (c1 and
-# c5: Scatter G=8, c2: Gather-1, c3: image Scatter, c4: Scatter G=2), from the full-size ncu captures
-# summarised under profiles/ (a profiler cannot run inside the timed region).
-NCU_TRAFFIC_BYTES = {"c1": 50432768 + 5723136, "c2": 279402240 + 99670016, "c3": 381974272 + 90594048,
-                     "c4": 1967612000 + 238374912, "c5": 6485108000 + 507752704}
+# c5: Scatter G=8, c2: Gather-1, c3: image Scatter, c4: Scatter G=2), from the full-size one-pass ncu captures
+# in profiles/attention_rows_kernel.md (a profiler cannot run inside the timed region).
+NCU_TRAFFIC_BYTES = {"c1": 50400000 + 2280000, "c2": 289110000 + 95040000, "c3": 403430000 + 89110000,
+                     "c4": 403290000 + 237260000, "c5": 853390000 + 503620000}
 DEFAULT_WORKLOAD = "c5"
 
 WORKLOADS = {
