@@ -71,3 +71,8 @@ lib = _load()
 
 def strerror(status: int) -> str:
     return lib.intra_b200_strerror(status).decode()
+
+
+def strides3(t) -> ctypes.Array:
+    """{batch, token, head} element strides of a (B, S, H, 128) tensor as int64[3]."""
+    return (ctypes.c_int64 * 3)(t.stride(0), t.stride(1), t.stride(2))
