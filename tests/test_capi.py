@@ -1,6 +1,8 @@
 """The C-ABI library loads, exports every symbol the public header declares, and rejects bad
 arguments before touching a GPU."""
+import ast
 import ctypes
+import importlib
 import os
 import re
 
@@ -144,3 +146,13 @@ def test_launcher_picks_the_kernel_form_by_item_length(lib):
         assert form(LLM, SCATTER, 65536, 8, 32, 8) == 4
     finally:
         assert lib.intra_b200_test_force_path(0, 0) == 0
+
+
+def test_names_bench_takes_from_the_package_exist():
+    """bench.py imports some of them inside the functions that only run on a GPU."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    names = [(node.module, name.name) for node in ast.walk(ast.parse(open(os.path.join(root, "bench.py")).read()))
+             if isinstance(node, ast.ImportFrom) and node.module.startswith("intra_b200") for name in node.names]
+    assert names
+    for module, name in names:
+        assert hasattr(importlib.import_module(module), name), f"{module} has no {name}"
