@@ -176,6 +176,8 @@ def test_a_failed_launch_is_reported_once(lib):
     q, k, v = _inputs(1, 32, 8, 100)
     want, out = decode_attn(q, k, v), torch.empty(1, 1, 32, 128, dtype=torch.bfloat16, device="cuda")
     prompt = torch.randn(1, 64, 4, 128, device="cuda").bfloat16()
+    with torch.no_grad():                            # a first attention call sets the device up, which forgets errors
+        prefill = intra_llm_attn(prompt, prompt, prompt, "window")
     stream = torch.cuda.Stream()
     torch.cuda.synchronize()
     rt = ctypes.CDLL("libcudart.so.%s" % torch.version.cuda.split(".")[0])        # the runtime torch has loaded
@@ -193,7 +195,7 @@ def test_a_failed_launch_is_reported_once(lib):
     rt.cudaGetLastError()
     assert rc == -4 and lib.intra_b200_last_cuda_error() != 0
     with torch.no_grad():
-        assert bool(torch.isfinite(intra_llm_attn(prompt, prompt, prompt, "window")).all())
+        assert torch.equal(intra_llm_attn(prompt, prompt, prompt, "window"), prefill)
     assert decode(None) == 0
     torch.cuda.synchronize()
     assert torch.equal(out, want)
